@@ -625,6 +625,8 @@ void free_far(hmg_matrix* h)
     dfree(h->ptrV, s);
     dfree(h->tbuf, s);
     dfree(h->far_list, s);
+    dfree(h->vt_tasks, s);
+    h->vt_large = h->vt_small = 0;
     dfree(h->tier32, s);
     dfree(h->tier16, s);
     h->h_r32.clear();
