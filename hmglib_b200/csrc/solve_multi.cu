@@ -207,6 +207,7 @@ struct hmg_cg_multi {
     int* flags = nullptr;  // active[k], then the bad flag
     MrScal s{};
     MrCheck checks[MR_INFLIGHT + 1];
+    char* pinned = nullptr;     // the checks' host buffers, one allocation (1.1 ms each)
     int nchecks = 0, head = 0;  // checks in flight: a queue in `checks`
     int state = MR_RESID;
     int iters = 0, outer = 0;
@@ -369,10 +370,8 @@ static void mr_free(hmg_cg_multi* c)
     dfree(c->part, s); dfree(c->sc, s); dfree(c->flags, s);
     for (MrCheck& ck : c->checks) {
         if (ck.ev) cudaEventDestroy(ck.ev);
-        if (ck.rr) cudaFreeHost(ck.rr);
-        if (ck.bb) cudaFreeHost(ck.bb);
-        if (ck.active) cudaFreeHost(ck.active);
     }
+    if (c->pinned) cudaFreeHost(c->pinned);
     delete c;
 }
 
@@ -485,16 +484,21 @@ hmg_status hmg_cg_multi_begin(hmg_cg_multi** out, hmg_matrix* h, int nrhs, doubl
     c->s = MrScal{c->sc, c->sc + 64, c->sc + 128, c->sc + 192, c->sc + 256, c->sc + 320, c->flags, c->flags + 64};
     // the bad flag sits after the k activity flags in the copies: keep it at flags[k]
     c->s.bad = c->flags + nrhs;
-    for (MrCheck& ck : c->checks) {
-        if (cudaEventCreateWithFlags(&ck.ev, cudaEventDisableTiming) != cudaSuccess ||
-            cudaMallocHost((void**)&ck.rr, sizeof(double) * 64) != cudaSuccess ||
-            cudaMallocHost((void**)&ck.bb, sizeof(double) * 64) != cudaSuccess ||
-            cudaMallocHost((void**)&ck.active, sizeof(int) * 65) != cudaSuccess) {
-            cudaGetLastError();
-            mr_free(c);
-            set_error("hmg_cg_multi_begin: cannot create events / pinned buffers");
-            return HMG_ERR_CUDA;
-        }
+    const size_t per = sizeof(double) * 128 + sizeof(int) * 66;
+    bool made = cudaMallocHost((void**)&c->pinned, per * (MR_INFLIGHT + 1)) == cudaSuccess;
+    if (!made) c->pinned = nullptr;
+    for (int i = 0; i <= MR_INFLIGHT && made; i++) {
+        MrCheck& ck = c->checks[i];
+        ck.rr = reinterpret_cast<double*>(c->pinned + per * i);
+        ck.bb = ck.rr + 64;
+        ck.active = reinterpret_cast<int*>(ck.bb + 64);
+        made = cudaEventCreateWithFlags(&ck.ev, cudaEventDisableTiming) == cudaSuccess;
+    }
+    if (!made) {
+        cudaGetLastError();
+        mr_free(c);
+        set_error("hmg_cg_multi_begin: cannot create events / pinned buffers");
+        return HMG_ERR_CUDA;
     }
     if (cudaMemsetAsync(c->flags, 0, sizeof(int) * 65, s) != cudaSuccess ||
         cudaMemsetAsync(c->sc, 0, sizeof(double) * 6 * 64, s) != cudaSuccess) {

@@ -8,6 +8,7 @@
 // up-front histogram of all eight digits), which is exact and removes the top
 // pass of 3D codes (60 significant bits).
 #include <cstdarg>
+#include <mutex>
 
 #include "radix.cuh"
 #include "util.cuh"
@@ -206,6 +207,65 @@ hmg_status radix_sort_pairs(uint64_t* keys, uint32_t* vals, int n, int key_bits,
     }
     dfree(hist, s); dfree(counts, s); dfree(k2, s); dfree(v2, s);
     return st;
+}
+
+// ---------------------------------------------------------------------------
+// the library's device pools
+// ---------------------------------------------------------------------------
+static constexpr int POOL_DEVICES = 64;
+static std::mutex g_pool_mutex;
+static cudaMemPool_t g_pool[POOL_DEVICES];
+static bool g_pool_tried[POOL_DEVICES];
+static int g_pool_users[POOL_DEVICES];  // live handles
+
+static cudaMemPool_t pool_of(int device)  // g_pool_mutex held
+{
+    if (device < 0 || device >= POOL_DEVICES) return nullptr;
+    if (!g_pool_tried[device]) {
+        g_pool_tried[device] = true;
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        if (cudaMemPoolCreate(&g_pool[device], &props) != cudaSuccess) {
+            cudaGetLastError();
+            g_pool[device] = nullptr;
+        }
+    }
+    return g_pool[device];
+}
+
+cudaMemPool_t device_pool()
+{
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    return pool_of(device);
+}
+
+// bytes the pool keeps mapped at a synchronisation
+static void pool_keep(cudaMemPool_t pool, unsigned long long bytes)
+{
+    if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &bytes) != cudaSuccess) cudaGetLastError();
+}
+
+void pool_retain(int device)
+{
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    const cudaMemPool_t pool = pool_of(device);
+    if (pool && g_pool_users[device]++ == 0) pool_keep(pool, POOL_KEEP);
+}
+
+void pool_release(int device)
+{
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    const cudaMemPool_t pool = pool_of(device);
+    if (!pool || --g_pool_users[device] > 0) return;
+    pool_keep(pool, 0);
+    if (cudaMemPoolTrimTo(pool, 0) != cudaSuccess) cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------

@@ -7,13 +7,27 @@
 
 namespace hmg {
 
-// Stream-ordered device allocation helpers (cudaMallocAsync pool).
+// The library's own stream-ordered pool on the current device (null if it cannot be
+// created: the device's default pool then serves).  While handles live it keeps up to
+// POOL_KEEP freed bytes mapped; the last handle's destruction gives them back.  The
+// default pool, which other code may share and whose settings stay untouched, unmaps
+// everything free at every synchronisation: about 0.2 ms to map and 0.2 ms to unmap a
+// small block, 6.3 ms a GB each way (measured on a B200), in a setup that synchronises
+// some twenty times.  Thread-safe.
+static constexpr unsigned long long POOL_KEEP = 1ull << 30;
+cudaMemPool_t device_pool();
+void pool_retain(int device);
+void pool_release(int device);
+
+// Stream-ordered device allocation helpers.
 template <typename T>
 hmg_status dalloc(T** p, size_t count, cudaStream_t s)
 {
     *p = nullptr;
     if (count == 0) count = 1;
-    cudaError_t e = cudaMallocAsync((void**)p, count * sizeof(T), s);
+    const cudaMemPool_t pool = device_pool();
+    cudaError_t e = pool ? cudaMallocFromPoolAsync((void**)p, count * sizeof(T), pool, s)
+                         : cudaMallocAsync((void**)p, count * sizeof(T), s);
     if (e != cudaSuccess) {
         cudaGetLastError();
         set_error("device allocation of %zu bytes failed: %s", count * sizeof(T),
