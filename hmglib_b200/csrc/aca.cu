@@ -1,11 +1,19 @@
-// aca.cu -- batched ACA of all admissible blocks, one CTA per block, FP64.
+// aca.cu -- batched ACA of all admissible blocks, FP64.
 //
 // The reference (linear_algebra.cu:3684-4012) advances all blocks in lock step:
 // every rank step is ~10 kernel launches, Thrust reduce_by_key calls and a host
-// synchronisation, over "batched" vectors that concatenate all blocks.  Here one
-// CTA owns one block for its whole ACA: the residual row / column, the pivot
-// searches and the norms are CTA reductions, and the only traffic is the block's
-// own U/V panels (L2-resident for all but the largest blocks).
+// synchronisation, over "batched" vectors that concatenate all blocks.  Here one CTA
+// (small blocks: one warp) owns one block for its whole ACA: the residual row / column,
+// the pivot searches and the norms are its reductions, and the only traffic is the
+// block's own terms.
+//
+// Bound by the latency of the rank steps (a chain of r FP64 multiply-adds and a kernel
+// entry, twice, with four barriers), not by bytes or FP64 rate: 30-50 % of issue slots
+// used.  Measured at N = 2^17 (uniform 3D, Matern, eps 1e-8, mean rank 48, 108k blocks):
+// 152 ms in the ACA kernels against 249 ms for a CTA of 256 threads (blocks to 512: a
+// warp) that kept every term in device memory and ran the cross terms at every step;
+// hmg_precompute_aca 190 ms against 575 (the rest: 16 GB of scratch in a pool that maps and
+// unmaps it, now 4 GB).  Factors and ranks are the same to the last bit.
 //
 // Two modes:
 //   * fixed (eps <= 0): the reference's semantics -- rank k_b = min(k,m1,m2)
@@ -28,14 +36,13 @@
 #include <cuda_fp8.h>
 
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "hmg_matrix.cuh"
 
 namespace hmg {
 
-static constexpr int ACA_THREADS = 256;
-static constexpr int ACA_WARPS = ACA_THREADS / 32;
 static constexpr int ACA_KMAX = 512;
 
 struct AcaBatch {
@@ -46,26 +53,14 @@ struct AcaBatch {
     double* V;
     int* rank_out;           // per batch entry
     double* s2_out;          // per batch entry: |U V^T|_F^2 (adaptive mode), may be null
+    const long long* soff;   // per batch entry: its first term among the batch's (mixed storage)
+    double* tnorm;           // per term |u_l|^2, |v_l|^2, max |u_l| (mixed storage, else null)
 };
 
 struct BlockGeom {
     const int *r0, *m1, *c0, *m2;
     const double* param;  // per-block kernel parameter (grouped H-matrices), else null
 };
-
-__device__ __forceinline__ double block_sum(double v, double* red)
-{
-    int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    __syncthreads();
-    if (lane == 0) red[warp] = v;
-    __syncthreads();
-    double s = 0.0;
-#pragma unroll
-    for (int w = 0; w < ACA_WARPS; w++) s += red[w];
-    return s;
-}
 
 // (value, index) argmax; last = true: ties go to the larger index, else the smaller.
 __device__ __forceinline__ bool better(double a, int i, double b, int j, bool last)
@@ -74,199 +69,420 @@ __device__ __forceinline__ bool better(double a, int i, double b, int j, bool la
     return last ? i > j : i < j;
 }
 
-__device__ __forceinline__ void block_argmax(double& a, int& i, bool last, double* reda,
-                                             int* redi)
+// The warp's entry of largest magnitude and its index (ties: the smaller index, or the
+// larger with `last`; a NaN counts as 0), by integer reductions of the magnitude's words
+// and the index: an FP64 compare-and-select butterfly takes five times the instructions.
+__device__ __forceinline__ void warp_argmax(double& v, int& i, bool last)
 {
-    int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        double b = __shfl_xor_sync(0xffffffffu, a, o);
-        int j = __shfl_xor_sync(0xffffffffu, i, o);
-        if (better(b, j, a, i, last)) { a = b; i = j; }
-    }
-    __syncthreads();
-    if (lane == 0) { reda[warp] = a; redi[warp] = i; }
-    __syncthreads();
-    a = reda[0];
-    i = redi[0];
-#pragma unroll
-    for (int w = 1; w < ACA_WARPS; w++)
-        if (better(reda[w], redi[w], a, i, last)) { a = reda[w]; i = redi[w]; }
+    const unsigned long long key = v == v ? (unsigned long long)__double_as_longlong(fabs(v)) : 0ull;
+    const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
+    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+    const bool in = hi == mh && lo == ml;
+    const int j = last ? __reduce_max_sync(0xffffffffu, in ? i : -1) : __reduce_min_sync(0xffffffffu, in ? i : 0x7fffffff);
+    const unsigned at = __ballot_sync(0xffffffffu, in && i == j);
+    v = __shfl_sync(0xffffffffu, v, at ? __ffs(at) - 1 : 0);
+    i = j;
 }
 
-// four CTAs an SM: the rank steps are latency-bound, so occupancy sets their pace
-__global__ void __launch_bounds__(ACA_THREADS, 4)
-k_aca(BlockGeom g, KernelSpec K0, PointsView P, AcaBatch B, int k, double eps, const int* elist)
+// c += A B of one 8 x 8 x 4 FP64 MMA: lane (g, t) has A[g][t], B[t][g], C[g][2t], C[g][2t+1]
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b)
 {
-    __shared__ double coef[ACA_KMAX];
-    __shared__ double red[ACA_WARPS];
-    __shared__ double reda[ACA_WARPS];
-    __shared__ int redi[ACA_WARPS];
-    extern __shared__ unsigned used[];  // adaptive mode: one bit per row
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+        : "+d"(c[0]), "+d"(c[1]) : "d"(a), "d"(b));
+}
 
-    const int e = elist ? elist[blockIdx.x] : blockIdx.x;
+// The share of warp w of nw in |sum_{l < r} u_l v_l^T|_F^2 = sum_{l, l'} (u_l . u_l')(v_l . v_l'):
+// the 8 x 8 products of pairs of 8 terms, every nw-th pair (b0 <= b1).  The warp's lanes hold
+// the parts of its sum.
+template <class FU, class FV>
+__device__ __forceinline__ double gram_share(int r, int m1, int m2, int w, int nw, FU term_u, FV term_v)
+{
+    const int lane = threadIdx.x & 31, nb = (r + 7) >> 3, g = lane >> 2, t = lane & 3;
+    double acc = 0.0;
+    int p = w;
+    for (int b0 = 0; b0 < nb; b0++) {
+        const int row = nb - b0;
+        for (; p < row; p += nw) {
+            const int b1 = b0 + p, l0 = 8 * b0 + g, l1 = 8 * b1 + g;
+            double cu[2] = {0.0, 0.0}, cv[2] = {0.0, 0.0};
+            const double *xu = l0 < r ? term_u(l0) : nullptr, *yu = l1 < r ? term_u(l1) : nullptr;
+            const double *xv = l0 < r ? term_v(l0) : nullptr, *yv = l1 < r ? term_v(l1) : nullptr;
+            for (int i0 = 0; i0 < m1; i0 += 4) {
+                const bool in = i0 + t < m1;
+                dmma(cu, xu && in ? xu[i0 + t] : 0.0, yu && in ? yu[i0 + t] : 0.0);
+            }
+            for (int i0 = 0; i0 < m2; i0 += 4) {
+                const bool in = i0 + t < m2;
+                dmma(cv, xv && in ? xv[i0 + t] : 0.0, yv && in ? yv[i0 + t] : 0.0);
+            }
+            acc += (b0 == b1 ? 1.0 : 2.0) * (cu[0] * cv[0] + cu[1] * cv[1]);
+        }
+        p -= row;
+    }
+    return acc;
+}
+
+// Kernel entries between one fixed point and the points of an array (SoA): the fixed
+// point's coordinates are loaded once.
+struct Entries {
+    const double *cx, *cy, *cz;  // the points (cz: null in 2D)
+    double fx, fy, fz;           // the fixed point
+    int same;                    // the index whose entry is on the diagonal (gets the regularization)
+    __device__ __forceinline__ Entries(const double* const* points, int p0, const double* const* fixed, int f, int dim, int d)
+        : cx(points[0] + p0), cy(points[1] + p0), cz(dim > 2 ? points[2] + p0 : nullptr), fx(fixed[0][f]), fy(fixed[1][f]),
+          fz(dim > 2 ? fixed[2][f] : 0.0), same(d)
+    {
+    }
+    __device__ __forceinline__ double operator()(const KernelSpec& K, int j) const
+    {
+        const double x = fx - cx[j], y = fy - cy[j];
+        double s = __fma_rn(x, x, 0.0);
+        s = __fma_rn(y, y, s);
+        if (cz) {
+            const double z = fz - cz[j];
+            s = __fma_rn(z, z, s);
+        }
+        const double v = kernel_from_sq(K, s);
+        return j == same ? v + K.reg : v;
+    }
+};
+
+// One block's ACA by one CTA of T threads.
+//
+// What a rank step reads is the block's earlier terms, twice: the residual of the pivot
+// row needs every earlier v_l, that of the pivot column every earlier u_l.  The first
+// `cap` terms (as many as the CTA's shared memory takes) are kept there, FP64 as in the
+// scratch, and only later ones are read back from the scratch.  The residuals add the
+// terms in order, one fused multiply-add each, wherever a term lies.
+//
+// The adaptive mode's third pass, the cross terms of |S_r|_F, is not run every step.
+// |S_r|_F is at most the sum of the terms' norms; while a term is larger than eps times
+// that bound the stopping test cannot hold.  When it no longer is, |S_r|_F^2 is computed
+// once from the Gram matrices of the terms (FP64 tensor-core products of 8 x 8 terms), and
+// updated exactly from there on (usually one to three steps).
+template <int T> struct AcaShared {
+    double v[T / 32], p[T / 32], q[T / 32], x[T / 32];
+    int i[T / 32];
+};
+
+template <int T, int C>
+struct AcaBlock {
+    static constexpr int NW = T / 32;
+    AcaShared<T>& sh;
+    double* sp;           // the terms in shared memory: ms doubles each, u_l then v_l
+    int ms, cap;
+    double *U, *V;        // the terms in the scratch
+    int m1, m2;
+    int tid, lane, warp;
+
+    __device__ __forceinline__ const double* term_u(int l) const { return l < cap ? sp + (size_t)l * ms : U + (size_t)l * m1; }
+    __device__ __forceinline__ const double* term_v(int l) const { return l < cap ? sp + (size_t)l * ms + m1 : V + (size_t)l * m2; }
+    // where entry j of v_r is kept until the pivot is known
+    __device__ __forceinline__ double* slot_v(int r) const { return r < cap ? sp + (size_t)r * ms + m1 : V + (size_t)r * m2; }
+
+    // val[q] = entry(idx[q]) - sum_l coef[l] term_l[idx[q]], l in order.  coef is 16-byte
+    // aligned.  Where most terms lie in the scratch (two entries a thread: the largest
+    // blocks), eight scratch loads an entry are in flight at any time, the first ones before
+    // the entries are evaluated.
+    template <int N, class F>
+    __device__ __forceinline__ void residual(double (&val)[N], const int (&idx)[N], F entry, const double* s0,
+                                             const double* g0, int ld, int r, const double* coef) const
+    {
+        constexpr bool AHEAD = C > 1;
+        const int rs = r < cap ? r : cap;
+        const double* g = g0 + (size_t)rs * ld;
+        double t[8][N];
+        if (AHEAD) {
+#pragma unroll
+            for (int u = 0; u < 8; u++)
+#pragma unroll
+                for (int q = 0; q < N; q++) t[u][q] = rs + u < r ? __ldcg(g + (size_t)u * ld + idx[q]) : 0.0;
+        }
+#pragma unroll
+        for (int q = 0; q < N; q++) val[q] = entry(idx[q]);
+        const double* sq[N];
+#pragma unroll
+        for (int q = 0; q < N; q++) sq[q] = s0 + idx[q];
+        int l = 0;
+        for (; l + 4 <= rs; l += 4) {
+            const double2 c0 = *reinterpret_cast<const double2*>(coef + l), c1 = *reinterpret_cast<const double2*>(coef + l + 2);
+#pragma unroll
+            for (int q = 0; q < N; q++) {
+                val[q] = __fma_rn(-c0.x, sq[q][0], val[q]);
+                val[q] = __fma_rn(-c0.y, sq[q][ms], val[q]);
+                val[q] = __fma_rn(-c1.x, sq[q][2 * ms], val[q]);
+                val[q] = __fma_rn(-c1.y, sq[q][3 * ms], val[q]);
+                sq[q] += 4 * ms;
+            }
+        }
+        for (; l < rs; l++)
+#pragma unroll
+            for (int q = 0; q < N; q++) {
+                val[q] = __fma_rn(-coef[l], *sq[q], val[q]);
+                sq[q] += ms;
+            }
+        if (AHEAD) {
+            for (; l < r; l += 8, g += 8 * (size_t)ld) {
+#pragma unroll
+                for (int u = 0; u < 8; u++) {
+                    if (l + u >= r) break;
+                    const double c = coef[l + u];
+#pragma unroll
+                    for (int q = 0; q < N; q++) val[q] = __fma_rn(-c, t[u][q], val[q]);
+                    if (l + u + 8 < r)
+#pragma unroll
+                        for (int q = 0; q < N; q++) t[u][q] = __ldcg(g + (size_t)(u + 8) * ld + idx[q]);
+                }
+            }
+        } else {
+            for (; l + 8 <= r; l += 8, g += 8 * (size_t)ld) {
+#pragma unroll
+                for (int u = 0; u < 8; u++)
+#pragma unroll
+                    for (int q = 0; q < N; q++) t[u][q] = __ldcg(g + (size_t)u * ld + idx[q]);
+#pragma unroll
+                for (int u = 0; u < 8; u++)
+#pragma unroll
+                    for (int q = 0; q < N; q++) val[q] = __fma_rn(-coef[l + u], t[u][q], val[q]);
+            }
+            for (; l < r; l++, g += ld)
+#pragma unroll
+                for (int q = 0; q < N; q++) val[q] = __fma_rn(-coef[l], __ldcg(g + idx[q]), val[q]);
+        }
+    }
+
+    // Residuals of the n entries of a row or column, each handed to take(index, value), a
+    // thread's own entry tid first: C at a time where the thread's warp has as many.
+    template <class F, class G>
+    __device__ __forceinline__ void residuals(int n, F entry, const double* s0, const double* g0, int ld, int r,
+                                              const double* coef, G take) const
+    {
+        for (int j = tid; j < n; j += C * T) {
+            if (C > 1 && (j & ~31) + T < n) {
+                const int idx[2] = {j, min(j + T, n - 1)};
+                double val[2];
+                residual<2>(val, idx, entry, s0, g0, ld, r, coef);
+                take(j, val[0]);
+                if (j + T < n) take(j + T, val[1]);
+            } else {
+                const int idx[1] = {j};
+                double val[1];
+                residual<1>(val, idx, entry, s0, g0, ld, r, coef);
+                take(j, val[0]);
+            }
+        }
+    }
+
+    // The CTA's entry of largest magnitude, and with SUMS the sums p, q and the maximum x;
+    // every thread gets the results.  One barrier; the shared entries are free again at the
+    // next.
+    template <bool SUMS>
+    __device__ __forceinline__ void reduce(double& v, int& i, double& p, double& q, double& x, bool last) const
+    {
+        warp_argmax(v, i, last);
+        if (SUMS)
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                p += __shfl_xor_sync(0xffffffffu, p, o);
+                q += __shfl_xor_sync(0xffffffffu, q, o);
+                x = fmax(x, __shfl_xor_sync(0xffffffffu, x, o));
+            }
+        if (lane == 0) {
+            sh.v[warp] = v;
+            sh.i[warp] = i;
+            if (SUMS) { sh.p[warp] = p; sh.q[warp] = q; sh.x[warp] = x; }
+        }
+        __syncthreads();
+        const int w0 = lane & (NW - 1);
+        v = sh.v[w0];
+        i = sh.i[w0];
+        warp_argmax(v, i, last);
+        if (SUMS) {
+            p = sh.p[w0]; q = sh.q[w0]; x = sh.x[w0];
+#pragma unroll
+            for (int o = NW / 2; o > 0; o >>= 1) {
+                p += __shfl_xor_sync(0xffffffffu, p, o);
+                q += __shfl_xor_sync(0xffffffffu, q, o);
+                x = fmax(x, __shfl_xor_sync(0xffffffffu, x, o));
+            }
+        }
+    }
+
+    // |sum_{l < r} u_l v_l^T|_F^2.  Barriers on both sides.
+    __device__ __noinline__ double frobenius2(int r) const
+    {
+        return total(gram_share(r, m1, m2, warp, NW, [&](int l) { return term_u(l); }, [&](int l) { return term_v(l); }));
+    }
+
+    // cross terms of the last of r + 1 terms with the r before: sum_l (u_r . u_l)(v_r . v_l)
+    __device__ __noinline__ double cross_terms(int r) const
+    {
+        const double *ur = term_u(r), *vr = term_v(r);
+        double acc = 0.0;
+        for (int l = warp; l < r; l += NW) {
+            const double *ul = term_u(l), *vl = term_v(l);
+            double x = 0.0, y = 0.0;
+            for (int i = lane; i < m1; i += 32) x = __fma_rn(ur[i], ul[i], x);
+            for (int j = lane; j < m2; j += 32) y = __fma_rn(vr[j], vl[j], y);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                x += __shfl_xor_sync(0xffffffffu, x, o);
+                y += __shfl_xor_sync(0xffffffffu, y, o);
+            }
+            if (lane == 0) acc += x * y;
+        }
+        return total(acc);
+    }
+
+    __device__ double total(double s) const
+    {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        __syncthreads();
+        if (lane == 0) sh.p[warp] = s;
+        __syncthreads();
+        s = sh.p[lane & (NW - 1)];
+#pragma unroll
+        for (int o = NW / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        __syncthreads();
+        return s;
+    }
+};
+
+template <int T, int C, int CTAS>
+__global__ void __launch_bounds__(T, CTAS)
+k_aca(BlockGeom g, KernelSpec K0, PointsView P, AcaBatch B, int k, double eps, const int* elist, int panel, int kc)
+{
+    __shared__ AcaShared<T> sh;
+    // panel doubles of terms, the pivot row's and column's coefficients (kc >= the largest
+    // rank), then (adaptive mode) one bit per row
+    extern __shared__ __align__(16) double aca_smem[];
+    double *coef = aca_smem + panel, *coef2 = coef + kc;
+
+    const int e = elist[blockIdx.x];
     const int b = B.blocks[e];
     KernelSpec K = K0;
     if (g.param) K.param = g.param[b];
     const int r0 = g.r0[b], m1 = g.m1[b], c0 = g.c0[b], m2 = g.m2[b];
     int kb = k < m1 ? k : m1;
     kb = kb < m2 ? kb : m2;
-    double* U = B.U + B.uoff[e];
-    double* V = B.V + B.voff[e];
     const int tid = threadIdx.x;
+    unsigned* used = reinterpret_cast<unsigned*>(coef2 + kc);
+    const AcaBlock<T, C> A{sh, aca_smem, m1 + m2, panel / (m1 + m2), B.U + B.uoff[e], B.V + B.voff[e], m1, m2,
+                        tid, tid & 31, tid >> 5};
     const bool adaptive = eps > 0.0;
     int rank = 0;
-    double S2 = 0.0;  // adaptive mode: squared Frobenius norm of the approximant
+    double S2 = 0.0;        // adaptive mode: squared Frobenius norm of the approximant
+    double norms = 0.0;     // sum of the terms' norms, an upper bound of |S|_F
+    bool have_s2 = false;
 
-    if (!adaptive) {
-        int ir = -1;
-        for (int r = 0; r < kb; r++) {
-            bool found = false;
-            for (;;) {
-                if (ir >= m1 - 1) break;
-                ir += 1;
-                for (int l = tid; l < r; l += ACA_THREADS) coef[l] = U[ir + (size_t)l * m1];
-                __syncthreads();
-                double ss = 0.0;
-                for (int j = tid; j < m2; j += ACA_THREADS) {
-                    double val = kernel_entry(K, P, r0 + ir, c0 + j);
-                    for (int l = 0; l < r; l++)
-                        val = __fma_rn(-coef[l], V[j + (size_t)l * m2], val);
-                    V[j + (size_t)r * m2] = val;
-                    ss += val * val;
-                }
-                double n2 = block_sum(ss, red);
-                if (sqrt(n2) >= 1.0e-13) { found = true; break; }
-                __syncthreads();
-            }
-            if (!found) break;
-            double best = -1.0;
-            int jr = 0;
-            for (int j = tid; j < m2; j += ACA_THREADS) {
-                double a = fabs(V[j + (size_t)r * m2]);
-                if (better(a, j, best, jr, true)) { best = a; jr = j; }
-            }
-            block_argmax(best, jr, true, reda, redi);
-            const double piv = V[jr + (size_t)r * m2];
-            __syncthreads();
-            for (int j = tid; j < m2; j += ACA_THREADS)
-                V[j + (size_t)r * m2] = V[j + (size_t)r * m2] / piv;
-            for (int l = tid; l < r; l += ACA_THREADS) coef[l] = V[jr + (size_t)l * m2];
-            __syncthreads();
-            for (int i = tid; i < m1; i += ACA_THREADS) {
-                double val = kernel_entry(K, P, r0 + i, c0 + jr);
-                for (int l = 0; l < r; l++) val = __fma_rn(-coef[l], U[i + (size_t)l * m1], val);
-                U[i + (size_t)r * m1] = val;
-            }
-            rank = r + 1;
-            __syncthreads();
-        }
-    } else {
-        const int nwords = (m1 + 31) >> 5;
-        for (int w = tid; w < nwords; w += ACA_THREADS) used[w] = 0u;
+    if (adaptive) {
+        for (int w = tid; w < ((m1 + 31) >> 5); w += T) used[w] = 0u;
         __syncthreads();
-        int ir = 0, nused = 0;
-        for (int r = 0; r < kb; r++) {
-            int jr = -1;
-            double piv = 0.0;
-            bool have = false;
-            for (;;) {
+    }
+    int ir = adaptive ? 0 : -1, nused = 0;
+    for (int r = 0; r < kb; r++) {
+        // ---- pivot row: the next usable row's residual, its largest entry
+        double piv = 0.0, none = 0.0, nosum = 0.0;
+        double mine = 0.0;  // the raw entry tid of v_r (the others wait in vr)
+        int jr = -1;
+        double* vr = A.slot_v(r);
+        for (;;) {
+            if (adaptive) {
                 if (tid == 0) used[ir >> 5] |= 1u << (ir & 31);
                 nused++;
-                for (int l = tid; l < r; l += ACA_THREADS) coef[l] = U[ir + (size_t)l * m1];
-                __syncthreads();
-                double best = -1.0;
-                int bj = 0x7fffffff;
-                for (int j = tid; j < m2; j += ACA_THREADS) {
-                    double val = kernel_entry(K, P, r0 + ir, c0 + j);
-                    for (int l = 0; l < r; l++)
-                        val = __fma_rn(-coef[l], V[j + (size_t)l * m2], val);
-                    V[j + (size_t)r * m2] = val;
-                    double a = fabs(val);
-                    if (better(a, j, best, bj, false)) { best = a; bj = j; }
-                }
-                block_argmax(best, bj, false, reda, redi);
-                if (best > 0.0) {
-                    jr = bj;
-                    have = true;
-                    break;
-                }
+            } else {
+                if (ir >= m1 - 1) break;
+                ir += 1;
+            }
+            for (int l = tid; l < r; l += T) coef[l] = A.term_u(l)[ir];
+            __syncthreads();
+            double bv = 0.0, ss = 0.0;
+            int bj = adaptive ? 0x7fffffff : -1;
+            const Entries row(P.c2, c0, P.c1, r0 + ir, K.dim, r0 + ir - c0);
+            A.residuals(m2, [&](int q) { return row(K, q); }, A.sp + m1, A.V, m2, r, coef, [&](int j, double v) {
+                if (j == tid) mine = v;
+                else vr[j] = v;
+                ss += v * v;
+                if (better(fabs(v), j, fabs(bv), bj, !adaptive)) { bv = v; bj = j; }
+            });
+            if (adaptive) A.template reduce<false>(bv, bj, ss, nosum, none, false);
+            else A.template reduce<true>(bv, bj, ss, nosum, none, true);
+            if (adaptive ? fabs(bv) > 0.0 : sqrt(ss) >= 1.0e-13) {
+                jr = bj;
+                piv = bv;
+                break;
+            }
+            __syncthreads();  // the reduction's entries and coef are used again
+            if (adaptive) {
                 // zero residual row: the next unused row in index order
                 int cand = 0x7fffffff;
-                for (int i = tid; i < m1; i += ACA_THREADS)
+                for (int i = tid; i < m1; i += T)
                     if (!((used[i >> 5] >> (i & 31)) & 1u)) { cand = i; break; }
-                double dummy = 0.0;
-                block_argmax(dummy, cand, false, reda, redi);
+                double z = 0.0;
+                A.template reduce<false>(z, cand, nosum, nosum, none, false);
+                __syncthreads();
                 if (cand == 0x7fffffff) break;
                 ir = cand;
-                __syncthreads();
             }
-            if (!have) break;
-            piv = V[jr + (size_t)r * m2];
-            __syncthreads();
-            double pv = 0.0;
-            for (int j = tid; j < m2; j += ACA_THREADS) {
-                double v = V[j + (size_t)r * m2] / piv;
-                V[j + (size_t)r * m2] = v;
-                pv += v * v;
-            }
-            for (int l = tid; l < r; l += ACA_THREADS) coef[l] = V[jr + (size_t)l * m2];
-            __syncthreads();
-            double pu = 0.0, bu = -1.0;
-            int bi = 0x7fffffff;
-            for (int i = tid; i < m1; i += ACA_THREADS) {
-                double val = kernel_entry(K, P, r0 + i, c0 + jr);
-                for (int l = 0; l < r; l++) val = __fma_rn(-coef[l], U[i + (size_t)l * m1], val);
-                U[i + (size_t)r * m1] = val;
-                pu += val * val;
-                if (!((used[i >> 5] >> (i & 31)) & 1u)) {
-                    double a = fabs(val);
-                    if (better(a, i, bu, bi, false)) { bu = a; bi = i; }
-                }
-            }
-            double nv2 = block_sum(pv, red);
-            double nu2 = block_sum(pu, red);
-            block_argmax(bu, bi, false, reda, redi);
-            // cross terms sum_l (u_r . U_l)(v_r . V_l): warp w takes columns l = w mod 8 whole
-            // (coalesced dot products, a fixed-order warp reduction), warp 0 sums the
-            // products over l in order.  Few registers per thread, so several CTAs share an SM.
-            {
-                const int warp = tid >> 5, lane = tid & 31;
-                const double* ur = U + (size_t)r * m1;
-                const double* vr = V + (size_t)r * m2;
-                for (int l = warp; l < r; l += ACA_WARPS) {
-                    const double* ul = U + (size_t)l * m1;
-                    const double* vl = V + (size_t)l * m2;
-                    double a = 0.0, c = 0.0;
-                    for (int i = lane; i < m1; i += 32) a = __fma_rn(ur[i], ul[i], a);
-                    for (int j = lane; j < m2; j += 32) c = __fma_rn(vr[j], vl[j], c);
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) {
-                        a += __shfl_xor_sync(0xffffffffu, a, o);
-                        c += __shfl_xor_sync(0xffffffffu, c, o);
-                    }
-                    if (lane == 0) coef[l] = a * c;
-                }
-                __syncthreads();
-                if (warp == 0) {
-                    double p = 0.0;
-                    for (int l = lane; l < r; l += 32) p += coef[l];
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
-                    if (lane == 0) red[0] = p;
-                }
-                __syncthreads();
-            }
-            const double cross = red[0];
-            __syncthreads();
-            S2 = S2 + 2.0 * cross + nu2 * nv2;
-            rank = r + 1;
-            if (sqrt(nu2 * nv2) <= eps * sqrt(fabs(S2))) break;
-            if (nused >= m1) break;
-            if (bi == 0x7fffffff) break;
-            ir = bi;
-            __syncthreads();
         }
+        if (jr < 0) break;
+        // ---- the row scaled by the pivot
+        for (int l = tid; l < r; l += T) coef2[l] = A.term_v(l)[jr];
+        double pv = 0.0;
+        for (int j = tid; j < m2; j += T) {
+            const double v = (j == tid ? mine : vr[j]) / piv;
+            if (r < A.cap) A.sp[(size_t)r * A.ms + m1 + j] = v;
+            A.V[j + (size_t)r * m2] = v;
+            pv += v * v;
+        }
+        __syncthreads();
+        // ---- pivot column: residual, norm, and (adaptive) its largest unused row
+        double pu = 0.0, bu = 0.0, mu = 0.0;
+        int bi = 0x7fffffff;
+        const Entries col(P.c1, r0, P.c2, c0 + jr, K.dim, c0 + jr - r0);
+        A.residuals(m1, [&](int q) { return col(K, q); }, A.sp, A.U, m1, r, coef2, [&](int i, double v) {
+            if (r < A.cap) A.sp[(size_t)r * A.ms + i] = v;
+            A.U[i + (size_t)r * m1] = v;
+            pu += v * v;
+            mu = fmax(mu, fabs(v));
+            if (adaptive && !((used[i >> 5] >> (i & 31)) & 1u) && better(fabs(v), i, fabs(bu), bi, false)) {
+                bu = v;
+                bi = i;
+            }
+        });
+        rank = r + 1;
+        if (!adaptive) {
+            __syncthreads();
+            continue;
+        }
+        A.template reduce<true>(bu, bi, pv, pu, mu, false);
+        __syncthreads();  // u_r, v_r complete; the reduction's entries are used again
+        if (B.tnorm && tid == 0) {
+            double* tn = B.tnorm + 3 * (B.soff[e] + r);
+            tn[0] = pu;
+            tn[1] = pv;
+            tn[2] = mu;
+        }
+        const double nn = sqrt(pu * pv);
+        norms += nn;
+        bool stop = false;
+        if (have_s2) {
+            const double cross = A.cross_terms(r);
+            S2 = S2 + 2.0 * cross + pu * pv;
+            stop = nn <= eps * sqrt(fabs(S2));
+        } else if (!(nn > eps * norms * (1.0 + 1e-12))) {
+            S2 = A.frobenius2(rank);
+            have_s2 = true;
+            stop = nn <= eps * sqrt(fabs(S2));
+        }
+        if (stop || nused >= m1 || bi == 0x7fffffff) break;
+        ir = bi;
+    }
+    if (adaptive && B.s2_out && !have_s2 && rank > 0) {
+        __syncthreads();
+        S2 = A.frobenius2(rank);
     }
     if (tid == 0) {
         B.rank_out[e] = rank;
@@ -274,16 +490,12 @@ k_aca(BlockGeom g, KernelSpec K0, PointsView P, AcaBatch B, int k, double eps, c
     }
 }
 
-
 // ---------------------------------------------------------------------------
 // The adaptive ACA of a small block (m1, m2 <= ACA_WSMALL) by one warp: the steps of
-// k_aca's adaptive mode with warp shuffles in place of CTA reductions and no CTA
-// barriers.  Most admissible blocks are small (at N = 2^20, 925k of 1.16M have
-// m1 + m2 < 512); a CTA of 256 threads per block would leave most lanes idle and
-// synchronise six times a rank step.
+// k_aca's adaptive mode with warp shuffles in place of CTA reductions and no CTA barriers.
 // ---------------------------------------------------------------------------
-static constexpr int ACA_WSMALL = 512;              // largest m1 and m2 of the warp variant
-static constexpr int ACA_WPC = 8;                   // warps (blocks) per CTA
+static constexpr int ACA_WSMALL = 128;  // largest m1 and m2 of the warp variant
+static constexpr int ACA_WPC = 8;       // warps (blocks) per CTA
 
 __device__ __forceinline__ double warp_sum(double v)
 {
@@ -292,15 +504,10 @@ __device__ __forceinline__ double warp_sum(double v)
     return v;
 }
 
-// (value, index) argmax over the warp; ties go to the smaller index
-__device__ __forceinline__ void warp_argmax_first(double& a, int& i)
+__device__ __noinline__ double warp_frobenius2(const double* U, const double* V, int m1, int m2, int r)
 {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const double b = __shfl_xor_sync(0xffffffffu, a, o);
-        const int j = __shfl_xor_sync(0xffffffffu, i, o);
-        if (better(b, j, a, i, false)) { a = b; i = j; }
-    }
+    return warp_sum(gram_share(r, m1, m2, 0, 1, [&](int l) { return U + (size_t)l * m1; },
+                               [&](int l) { return V + (size_t)l * m2; }));
 }
 
 __global__ void __launch_bounds__(ACA_WPC * 32, 4)
@@ -325,26 +532,29 @@ k_aca_warp(BlockGeom g, KernelSpec K0, PointsView P, AcaBatch B, int k, double e
     for (int w = lane; w < ACA_WSMALL / 32; w += 32) used[w] = 0u;
     __syncwarp();
     int rank = 0, ir = 0, nused = 0;
-    double S2 = 0.0;
+    double S2 = 0.0, norms = 0.0;  // as in k_aca
+    bool have_s2 = false;
     for (int r = 0; r < kb; r++) {
         int jr = -1;
+        double piv = 0.0;
         bool have = false;
         for (;;) {
             if (lane == 0) used[ir >> 5] |= 1u << (ir & 31);
             nused++;
             for (int l = lane; l < r; l += 32) coef[l] = U[ir + (size_t)l * m1];
             __syncwarp();
-            double best = -1.0;
+            double best = 0.0;
             int bj = 0x7fffffff;
+            const Entries row(P.c2, c0, P.c1, r0 + ir, K.dim, r0 + ir - c0);
             for (int j = lane; j < m2; j += 32) {
-                double val = kernel_entry(K, P, r0 + ir, c0 + j);
+                double val = row(K, j);
                 for (int l = 0; l < r; l++) val = __fma_rn(-coef[l], V[j + (size_t)l * m2], val);
                 V[j + (size_t)r * m2] = val;
-                const double a = fabs(val);
-                if (better(a, j, best, bj, false)) { best = a; bj = j; }
+                if (better(fabs(val), j, fabs(best), bj, false)) { best = val; bj = j; }
             }
-            warp_argmax_first(best, bj);
-            if (best > 0.0) {
+            warp_argmax(best, bj, false);
+            if (fabs(best) > 0.0) {
+                piv = best;
                 jr = bj;
                 have = true;
                 break;
@@ -354,14 +564,13 @@ k_aca_warp(BlockGeom g, KernelSpec K0, PointsView P, AcaBatch B, int k, double e
             for (int i = lane; i < m1; i += 32)
                 if (!((used[i >> 5] >> (i & 31)) & 1u)) { cand = i; break; }
             double dummy = 0.0;
-            warp_argmax_first(dummy, cand);
+            warp_argmax(dummy, cand, false);
             if (cand == 0x7fffffff) break;
             ir = cand;
             __syncwarp();
         }
         if (!have) break;
         __syncwarp();  // every lane's V[., r] written
-        const double piv = V[jr + (size_t)r * m2];
         double pv = 0.0;
         for (int j = lane; j < m2; j += 32) {
             const double v = V[j + (size_t)r * m2] / piv;
@@ -371,77 +580,130 @@ k_aca_warp(BlockGeom g, KernelSpec K0, PointsView P, AcaBatch B, int k, double e
         __syncwarp();
         for (int l = lane; l < r; l += 32) coef[l] = V[jr + (size_t)l * m2];
         __syncwarp();
-        double pu = 0.0, bu = -1.0;
+        double pu = 0.0, bu = 0.0, mu = 0.0;
+        const Entries col(P.c1, r0, P.c2, c0 + jr, K.dim, c0 + jr - r0);
         int bi = 0x7fffffff;
         for (int i = lane; i < m1; i += 32) {
-            double val = kernel_entry(K, P, r0 + i, c0 + jr);
+            double val = col(K, i);
             for (int l = 0; l < r; l++) val = __fma_rn(-coef[l], U[i + (size_t)l * m1], val);
             U[i + (size_t)r * m1] = val;
             pu += val * val;
-            if (!((used[i >> 5] >> (i & 31)) & 1u)) {
-                const double a = fabs(val);
-                if (better(a, i, bu, bi, false)) { bu = a; bi = i; }
-            }
+            mu = fmax(mu, fabs(val));
+            if (!((used[i >> 5] >> (i & 31)) & 1u) && better(fabs(val), i, fabs(bu), bi, false)) { bu = val; bi = i; }
         }
         const double nv2 = warp_sum(pv), nu2 = warp_sum(pu);
-        warp_argmax_first(bu, bi);
+        warp_argmax(bu, bi, false);
         __syncwarp();  // every lane's U[., r] written
-        // cross terms sum_l (u_r . U_l)(v_r . V_l), in l order
-        double cross = 0.0;
-        const double* ur = U + (size_t)r * m1;
-        const double* vr = V + (size_t)r * m2;
-        for (int l = 0; l < r; l++) {
-            const double* ul = U + (size_t)l * m1;
-            const double* vl = V + (size_t)l * m2;
-            double a = 0.0, c = 0.0;
-            for (int i = lane; i < m1; i += 32) a = __fma_rn(ur[i], ul[i], a);
-            for (int j = lane; j < m2; j += 32) c = __fma_rn(vr[j], vl[j], c);
-            cross += warp_sum(a) * warp_sum(c);
+        if (B.tnorm) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) mu = fmax(mu, __shfl_xor_sync(0xffffffffu, mu, o));
+            if (lane == 0) {
+                double* tn = B.tnorm + 3 * (B.soff[e] + r);
+                tn[0] = nu2;
+                tn[1] = nv2;
+                tn[2] = mu;
+            }
         }
-        S2 = S2 + 2.0 * cross + nu2 * nv2;
         rank = r + 1;
-        if (sqrt(nu2 * nv2) <= eps * sqrt(fabs(S2))) break;
+        const double nn = sqrt(nu2 * nv2);
+        norms += nn;
+        if (have_s2) {
+            // cross terms sum_l (u_r . U_l)(v_r . V_l), in l order
+            double cross = 0.0;
+            const double* ur = U + (size_t)r * m1;
+            const double* vr = V + (size_t)r * m2;
+            for (int l = 0; l < r; l++) {
+                const double* ul = U + (size_t)l * m1;
+                const double* vl = V + (size_t)l * m2;
+                double a = 0.0, c = 0.0;
+                for (int i = lane; i < m1; i += 32) a = __fma_rn(ur[i], ul[i], a);
+                for (int j = lane; j < m2; j += 32) c = __fma_rn(vr[j], vl[j], c);
+                cross += warp_sum(a) * warp_sum(c);
+            }
+            S2 = S2 + 2.0 * cross + nu2 * nv2;
+            if (nn <= eps * sqrt(fabs(S2))) break;
+        } else if (!(nn > eps * norms * (1.0 + 1e-12))) {
+            S2 = warp_frobenius2(U, V, m1, m2, rank);
+            have_s2 = true;
+            if (nn <= eps * sqrt(fabs(S2))) break;
+        }
         if (nused >= m1) break;
         if (bi == 0x7fffffff) break;
         ir = bi;
         __syncwarp();
     }
+    if (B.s2_out && !have_s2 && rank > 0) S2 = warp_frobenius2(U, V, m1, m2, rank);
     if (lane == 0) {
         B.rank_out[e] = rank;
         if (B.s2_out) B.s2_out[e] = S2;
     }
 }
 
+// Classes of blocks by their longer side: a thread an entry, and as much shared memory for
+// terms as leaves several CTAs an SM, whose rank steps (four barriers, an FP64 kernel entry
+// and two chains of dependent FP64 multiply-adds each) overlap: 52 KB hold 40 terms of a
+// 64 + 96 block, four CTAs to an SM.  Fewer threads than entries leave too few warps for the
+// FP64 latencies (128 threads for blocks of 129 to 256: 62 ms against 38 ms at N = 2^17).
+// Above 512 most terms lie in the scratch: two entries a thread keep sixteen loads in flight
+// each, which takes the registers of a whole SM (with half of them: 111 ms against 79).
+struct AcaClass {
+    int side;      // longest m1 or m2
+    int panel;     // bytes of terms in shared memory (the largest class: the row mask included)
+};
+static constexpr int ACA_NCLASS = 4;
+static constexpr AcaClass ACA_CLASSES[ACA_NCLASS] = {{128, 52 << 10}, {256, 72 << 10}, {512, 104 << 10}, {0x7fffffff, 208 << 10}};
+
+template <int T, int C, int CTAS>
+static hmg_status launch_aca(BlockGeom g, const KernelSpec& K, const PointsView& P, const AcaBatch& B, int k, double eps,
+                             const int* list, int n, int panel_bytes, int kc, int mask_bytes, cudaStream_t s)
+{
+    if (n == 0) return HMG_OK;
+    const int dyn = panel_bytes + 16 * kc + mask_bytes;
+    HMG_CUDA_TRY(cudaFuncSetAttribute(k_aca<T, C, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
+    k_aca<T, C, CTAS><<<n, T, dyn, s>>>(g, K, P, B, k, eps, list, panel_bytes / 8, kc);
+    HMG_LAUNCH_CHECK();
+    return HMG_OK;
+}
+
+// The smallest class: a warp a block in the adaptive mode, whose ranks there are small
+static hmg_status launch_small(BlockGeom g, const KernelSpec& K, const PointsView& P, const AcaBatch& B, int k, double eps,
+                               const int* list, int n, int kc, int mask_bytes, cudaStream_t s)
+{
+    if (eps <= 0.0) return launch_aca<128, 1, 4>(g, K, P, B, k, eps, list, n, ACA_CLASSES[0].panel, kc, mask_bytes, s);
+    if (n == 0) return HMG_OK;
+    k_aca_warp<<<ceil_div(n, ACA_WPC), ACA_WPC * 32, 0, s>>>(g, K, P, B, k, eps, list, n);
+    HMG_LAUNCH_CHECK();
+    return HMG_OK;
+}
+
 // Write the FP64 scratch factors of one block into its final storage:
 // U as tile slices (s_pad x r column-major, padding rows zero) and V^T as r rows
 // of m2p entries (padding zero).
+// A warp takes whole rows (of V^T) and whole columns of a tile slice (of U).
 template <typename T>
-__global__ void k_aca_compact(BlockGeom g, AcaBatch B, const int* tile_r0, const int* tile_s,
-                              const int* tile_pstart, const int* tfirst, const int* tlast,
-                              T* const* ptrU, T* const* ptrV)
+__global__ void __launch_bounds__(256) k_aca_compact(BlockGeom g, AcaBatch B, const int* tile_r0, const int* tile_s,
+                                                     const int* tile_pstart, const int* tfirst, const int* tlast,
+                                                     T* const* ptrU, T* const* ptrV)
 {
     const int e = blockIdx.x;
     const int b = B.blocks[e];
     const int r0 = g.r0[b], m1 = g.m1[b], m2 = g.m2[b];
     const int r = B.rank_out[e];
     if (r == 0) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const double* U = B.U + B.uoff[e];
     const double* V = B.V + B.voff[e];
     T* dU = ptrU[b];
     T* dV = ptrV[b];
     const int m2p = (m2 + 3) & ~3;
-    for (long long idx = threadIdx.x; idx < (long long)r * m2p; idx += blockDim.x) {
-        int l = (int)(idx / m2p), j = (int)(idx % m2p);
-        dV[idx] = j < m2 ? (T)V[j + (size_t)l * m2] : (T)0;
-    }
+    for (int l = warp; l < r; l += 8)
+        for (int j = lane; j < m2p; j += 32) dV[(size_t)l * m2p + j] = j < m2 ? (T)V[j + (size_t)l * m2] : (T)0;
     const int p0 = tile_pstart[tfirst[b]];
     for (int t = tfirst[b]; t <= tlast[b]; t++) {
-        int s = tile_s[t], sp = (s + 3) & ~3, tr = tile_r0[t] - r0;
+        const int s = tile_s[t], sp = (s + 3) & ~3, tr = tile_r0[t] - r0;
         T* dst = dU + (size_t)(tile_pstart[t] - p0) * r;
-        for (int idx = threadIdx.x; idx < sp * r; idx += blockDim.x) {
-            int l = idx / sp, i = idx % sp;
-            dst[idx] = i < s ? (T)U[(size_t)l * m1 + tr + i] : (T)0;
-        }
+        for (int l = warp; l < r; l += 8)
+            for (int i = lane; i < sp; i += 32) dst[(size_t)l * sp + i] = i < s ? (T)U[(size_t)l * m1 + tr + i] : (T)0;
     }
 }
 
@@ -471,72 +733,50 @@ struct TierOut {
     float* sv;         // per term: scale of v_l
 };
 
-__global__ void __launch_bounds__(256) k_aca_tiers(BlockGeom g, AcaBatch B, TierOut T)
+// One warp per block: the tiers and scales from the terms' norms.
+__global__ void __launch_bounds__(256) k_aca_tiers(AcaBatch B, TierOut T, int ne)
 {
-    __shared__ double sig[ACA_KMAX];
-    __shared__ double mu[ACA_KMAX];
-    __shared__ double mv[ACA_KMAX];
-    const int e = blockIdx.x;
-    const int b = B.blocks[e];
-    const int m1 = g.m1[b], m2 = g.m2[b];
+    const int e = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (e >= ne) return;
     const int r = B.rank_out[e];
-    const double* U = B.U + B.uoff[e];
-    const double* V = B.V + B.voff[e];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int l = warp; l < r; l += 8) {
-        double su = 0.0, mx_u = 0.0, sv = 0.0, mx_v = 0.0;
-        for (int i = lane; i < m1; i += 32) {
-            double u = U[(size_t)l * m1 + i];
-            su = fma(u, u, su);
-            mx_u = fmax(mx_u, fabs(u));
+    const double S = sqrt(fmax(B.s2_out[e], 0.0));
+    const long long so = T.soff[e];
+    const double* tn = B.tnorm + 3 * so;
+    // the tails, added from the last term on (32 terms at a time, an in-order scan)
+    int s16 = r, s8 = r;
+    double tail = 0.0;
+    for (int l1 = r; l1 > 0; l1 -= 32) {
+        const int l = l1 - 1 - lane;
+        const double sig = l >= 0 ? sqrt(tn[3 * l]) * sqrt(tn[3 * l + 1]) : 0.0;
+        double mine = 0.0;
+        for (int o = 0; o < 32; o++) {
+            tail += __shfl_sync(0xffffffffu, sig, o);
+            if (o == lane) mine = tail;
         }
-        for (int j = lane; j < m2; j += 32) {
-            double v = V[(size_t)l * m2 + j];
-            sv = fma(v, v, sv);
-            mx_v = fmax(mx_v, fabs(v));
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-            su += __shfl_xor_sync(0xffffffffu, su, o);
-            sv += __shfl_xor_sync(0xffffffffu, sv, o);
-            mx_u = fmax(mx_u, __shfl_xor_sync(0xffffffffu, mx_u, o));
-            mx_v = fmax(mx_v, __shfl_xor_sync(0xffffffffu, mx_v, o));
-        }
-        if (lane == 0) {
-            sig[l] = sqrt(su) * sqrt(sv);
-            mu[l] = mx_u;
-            mv[l] = mx_v;
-        }
+        const bool ok16 = l >= 0 && mine <= TAU16 * S, ok8 = l >= 0 && mine <= TAU8 * S;
+        const unsigned m16 = __ballot_sync(0xffffffffu, ok16), m8 = __ballot_sync(0xffffffffu, ok8);
+        if (m16) s16 = l1 - 1 - (31 - __clz(m16));
+        if (m8) s8 = l1 - 1 - (31 - __clz(m8));
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const double S = sqrt(fmax(B.s2_out[e], 0.0));
-        int s16 = r, s8 = r;
-        double tail = 0.0;
-        for (int l = r - 1; l >= 0; l--) {
-            tail += sig[l];
-            if (tail <= TAU16 * S) s16 = l;
-            if (tail <= TAU8 * S) s8 = l;
-        }
-        if (s8 < s16) s8 = s16;
-        s8 = r - ((r - s8) & ~3);          // FP8 terms: a multiple of 4
-        s16 = s8 - ((s8 - s16) & ~1);      // FP16 terms: a multiple of 2
+    if (s8 < s16) s8 = s16;
+    s8 = r - ((r - s8) & ~3);          // FP8 terms: a multiple of 4
+    s16 = s8 - ((s8 - s16) & ~1);      // FP16 terms: a multiple of 2
+    if (lane == 0) {
         T.r32[e] = s16;
         T.r16[e] = s8 - s16;
-        const long long so = T.soff[e];
-        for (int l = 0; l < r; l++) {
-            float a = 1.0f, c = 1.0f;
-            if (l >= s8) {
-                a = (float)(mu[l] / 448.0);
-                c = (float)(mv[l] / 448.0);
-            } else if (l >= s16) {
-                a = (float)mu[l];
-                c = (float)mv[l];
-            }
-            if (!(a > 0.0f)) a = 1.0f;
-            if (!(c > 0.0f)) c = 1.0f;
-            T.su[so + l] = a;
-            T.sv[so + l] = c;
+    }
+    // v_l's largest entry is its pivot, 1
+    for (int l = lane; l < r; l += 32) {
+        float a = 1.0f, c = 1.0f;
+        if (l >= s8) {
+            a = (float)(tn[3 * l + 2] / 448.0);
+            c = (float)(1.0 / 448.0);
+        } else if (l >= s16) {
+            a = (float)tn[3 * l + 2];
         }
+        if (!(a > 0.0f)) a = 1.0f;
+        T.su[so + l] = a;
+        T.sv[so + l] = c;
     }
 }
 
@@ -561,53 +801,66 @@ k_aca_compact_mixed(BlockGeom g, AcaBatch B, TierOut T, const int* tile_r0, cons
     const double* U = B.U + B.uoff[e];
     const double* V = B.V + B.voff[e];
     const int m2p = (m2 + 3) & ~3;
-    // V^T
-    float* v32 = static_cast<float*>(ptrV[b]);
-    __half* v16 = reinterpret_cast<__half*>(v32 + (size_t)r32 * m2p);
-    __nv_fp8_storage_t* v8 = reinterpret_cast<__nv_fp8_storage_t*>(v16 + (size_t)r16 * m2p);
-    float* scal = reinterpret_cast<float*>(v8 + (size_t)r8 * m2p);
-    for (long long idx = threadIdx.x; idx < (long long)r32 * m2p; idx += blockDim.x) {
-        const int l = (int)(idx / m2p), j = (int)(idx % m2p);
-        v32[idx] = j < m2 ? (float)V[j + (size_t)l * m2] : 0.0f;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // dst[0 .. rows): the storage words of a word column -- FP32, FP16 pairs or FP8 quads --
+    // from term l0 on, rows n.. zero (src + l ld: term l; sc: the terms' scales).  Four
+    // entries a lane at a time, so that their loads overlap.
+    auto convert = [&](uint32_t* dst, int rows, const double* src, size_t ld, int l0, int kind, int n, const float* sc) {
+        src += (size_t)l0 * ld;
+        const int nt = 1 << kind;
+        double q[4];
+#pragma unroll
+        for (int t = 0; t < 4; t++) q[t] = kind > 0 && t < nt ? (double)sc[l0 + t] : 1.0;
+        for (int i0 = lane; i0 < rows; i0 += 128) {
+            double x[4][4];
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+#pragma unroll
+                for (int t = 0; t < 4; t++) x[u][t] = t < nt && i0 + 32 * u < n ? src[(size_t)t * ld + i0 + 32 * u] : 0.0;
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                if (i0 + 32 * u >= rows) break;
+                uint32_t w;
+                if (kind == 0) {
+                    w = __float_as_uint((float)x[u][0]);
+                } else if (kind == 1) {
+                    const __half2 h = __halves2half2(__float2half_rn((float)(x[u][0] / q[0])), __float2half_rn((float)(x[u][1] / q[1])));
+                    w = *reinterpret_cast<const uint32_t*>(&h);
+                } else {
+                    w = 0u;
+#pragma unroll
+                    for (int t = 0; t < 4; t++)
+                        w |= (uint32_t)__nv_cvt_float_to_fp8((float)(x[u][t] / q[t]), __NV_SATFINITE, __NV_E4M3) << (8 * t);
+                }
+                dst[i0 + 32 * u] = w;
+            }
+        }
+    };
+    // word column c of a block: its tier and first term
+    auto column = [&](int c, int& kind, int& l0) {
+        kind = c < r32 ? 0 : (c < r32 + (r16 >> 1) ? 1 : 2);
+        l0 = kind == 0 ? c : (kind == 1 ? r32 + 2 * (c - r32) : r32 + r16 + 4 * (c - r32 - (r16 >> 1)));
+    };
+    const int nc = r32 + (r16 >> 1) + (r8 >> 2);
+    uint32_t* vw = reinterpret_cast<uint32_t*>(ptrV[b]);
+    for (int c = warp; c < nc; c += 8) {
+        int kind, l0;
+        column(c, kind, l0);
+        convert(vw + (size_t)c * m2p, m2p, V, m2, l0, kind, m2, T.sv + so);
     }
-    for (long long idx = threadIdx.x; idx < (long long)r16 * m2p; idx += blockDim.x) {
-        const int t = (int)(idx & 1), j = (int)((idx >> 1) % m2p), gp = (int)((idx >> 1) / m2p);
-        const int l = r32 + 2 * gp + t;
-        const float v = j < m2 ? (float)(V[j + (size_t)l * m2] / (double)T.sv[so + l]) : 0.0f;
-        v16[idx] = __float2half_rn(v);
-    }
-    for (long long idx = threadIdx.x; idx < (long long)r8 * m2p; idx += blockDim.x) {
-        const int t = (int)(idx & 3), j = (int)((idx >> 2) % m2p), gq = (int)((idx >> 2) / m2p);
-        const int l = r32 + r16 + 4 * gq + t;
-        const float v = j < m2 ? (float)(V[j + (size_t)l * m2] / (double)T.sv[so + l]) : 0.0f;
-        v8[idx] = __nv_cvt_float_to_fp8(v, __NV_SATFINITE, __NV_E4M3);
-    }
+    float* scal = reinterpret_cast<float*>(vw + (size_t)nc * m2p);
     for (int l = threadIdx.x; l < r; l += blockDim.x) scal[l] = T.su[so + l] * T.sv[so + l];
     // U tile slices
-    const int bpr = 4 * r32 + 2 * r16 + r8;
+    const int bpr = 4 * nc;
     const int p0 = tile_pstart[tfirst[b]];
     char* ubase = static_cast<char*>(ptrU[b]);
     for (int t = tfirst[b]; t <= tlast[b]; t++) {
         const int s = tile_s[t], sp = (s + 3) & ~3, tr = tile_r0[t] - r0;
-        char* slice = ubase + (size_t)(tile_pstart[t] - p0) * bpr;
-        float* u32 = reinterpret_cast<float*>(slice);
-        __half* u16 = reinterpret_cast<__half*>(slice + (size_t)sp * 4 * r32);
-        __nv_fp8_storage_t* u8 = reinterpret_cast<__nv_fp8_storage_t*>(slice + (size_t)sp * (4 * r32 + 2 * r16));
-        for (int idx = threadIdx.x; idx < sp * r32; idx += blockDim.x) {
-            const int l = idx / sp, i = idx % sp;
-            u32[idx] = i < s ? (float)U[(size_t)l * m1 + tr + i] : 0.0f;
-        }
-        for (int idx = threadIdx.x; idx < sp * r16; idx += blockDim.x) {
-            const int q = idx & 1, i = (idx >> 1) % sp, gp = (idx >> 1) / sp;
-            const int l = r32 + 2 * gp + q;
-            const float u = i < s ? (float)(U[(size_t)l * m1 + tr + i] / (double)T.su[so + l]) : 0.0f;
-            u16[idx] = __float2half_rn(u);
-        }
-        for (int idx = threadIdx.x; idx < sp * r8; idx += blockDim.x) {
-            const int q = idx & 3, i = (idx >> 2) % sp, gq = (idx >> 2) / sp;
-            const int l = r32 + r16 + 4 * gq + q;
-            const float u = i < s ? (float)(U[(size_t)l * m1 + tr + i] / (double)T.su[so + l]) : 0.0f;
-            u8[idx] = __nv_cvt_float_to_fp8(u, __NV_SATFINITE, __NV_E4M3);
+        uint32_t* slice = reinterpret_cast<uint32_t*>(ubase + (size_t)(tile_pstart[t] - p0) * bpr);
+        for (int c = warp; c < nc; c += 8) {
+            int kind, l0;
+            column(c, kind, l0);
+            convert(slice + (size_t)c * sp, sp, U + tr, m1, l0, kind, s, T.su + so);
         }
     }
 }
@@ -671,7 +924,7 @@ hmg_status run_aca(hmg_matrix* h, int k, double eps, int precision)
     size_t free_b = 0, total_b = 0;
     HMG_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
     size_t budget = free_b / 4;
-    if (budget > ((size_t)16 << 30)) budget = (size_t)16 << 30;
+    if (budget > ((size_t)4 << 30)) budget = (size_t)4 << 30;
     if (budget < ((size_t)64 << 20)) budget = (size_t)64 << 20;
 
     BlockGeom g{h->blk_r0, h->blk_m1, h->blk_c0, h->blk_m2, h->blk_param};
@@ -683,19 +936,39 @@ hmg_status run_aca(hmg_matrix* h, int k, double eps, int precision)
     P.n1 = h->n[0];
     P.n2 = h->n[1];
 
-    // Scratch of the batches, grown to the largest batch and reused across batches: the
-    // stream-ordered pool hands freed memory back at every synchronisation, so
-    // allocating it per batch would map gigabytes afresh for each one.
+    // Scratch of the batches, grown to the largest batch and reused across batches.  The
+    // factors' part is up to 4 GB, which the stream-ordered pool maps and unmaps at 6.3 ms a
+    // GB each way, cudaMalloc and cudaFree at 0.2 and 0.6 (measured): beyond what the pool
+    // keeps it comes from cudaMalloc.
+    static constexpr size_t POOL_SCRATCH = POOL_KEEP / 8 / sizeof(double);
     int* d_idx = nullptr;
     long long *d_uo = nullptr, *d_vo = nullptr, *d_so = nullptr;
-    double *dU = nullptr, *dV = nullptr, *d_s2 = nullptr;
+    double *dU = nullptr, *dV = nullptr, *d_s2 = nullptr, *d_tn = nullptr;
     int *d_rank = nullptr, *d_r32 = nullptr, *d_r16 = nullptr, *d_list = nullptr;
     float *d_su = nullptr, *d_sv = nullptr;
     size_t cap_ne = 0, cap_u = 0, cap_v = 0, cap_sc = 0;
+    auto drop = [&](double*& p, size_t cap) {
+        if (cap <= POOL_SCRATCH) dfree(p, s);
+        else if (p) cudaFree(p);
+        p = nullptr;
+    };
+    auto grow = [&](double*& p, size_t& cap, size_t n) {
+        drop(p, cap);
+        cap = n > 0 ? n : 1;
+        if (cap <= POOL_SCRATCH) return dalloc(&p, cap, s);
+        const cudaError_t e = cudaMalloc((void**)&p, cap * sizeof(double));
+        if (e == cudaSuccess) return HMG_OK;
+        cudaGetLastError();
+        p = nullptr;
+        set_error("allocating %zu bytes of ACA scratch failed: %s", cap * sizeof(double), cudaGetErrorString(e));
+        return e == cudaErrorMemoryAllocation ? HMG_ERR_NOMEM : HMG_ERR_CUDA;
+    };
     auto free_batch = [&]() {
-        dfree(d_idx, s); dfree(d_uo, s); dfree(d_vo, s); dfree(dU, s); dfree(dV, s);
+        drop(dU, cap_u);
+        drop(dV, cap_v);
+        dfree(d_idx, s); dfree(d_uo, s); dfree(d_vo, s);
         dfree(d_rank, s); dfree(d_s2, s); dfree(d_so, s); dfree(d_r32, s); dfree(d_r16, s);
-        dfree(d_su, s); dfree(d_sv, s); dfree(d_list, s);
+        dfree(d_su, s); dfree(d_sv, s); dfree(d_tn, s); dfree(d_list, s);
         cap_ne = cap_u = cap_v = cap_sc = 0;
     };
     int bstart = h->ndense;
@@ -738,17 +1011,13 @@ hmg_status run_aca(hmg_matrix* h, int k, double eps, int precision)
             }
         }
         if ((size_t)us > cap_u) {
-            dfree(dU, s);
-            cap_u = (size_t)us;
-            if ((st = dalloc(&dU, cap_u, s))) {
+            if ((st = grow(dU, cap_u, (size_t)us))) {
                 free_batch();
                 return st;
             }
         }
         if ((size_t)vs > cap_v) {
-            dfree(dV, s);
-            cap_v = (size_t)vs;
-            if ((st = dalloc(&dV, cap_v, s))) {
+            if ((st = grow(dV, cap_v, (size_t)vs))) {
                 free_batch();
                 return st;
             }
@@ -756,8 +1025,9 @@ hmg_status run_aca(hmg_matrix* h, int k, double eps, int precision)
         if (mixed && (size_t)nscale > cap_sc) {
             dfree(d_su, s);
             dfree(d_sv, s);
+            dfree(d_tn, s);
             cap_sc = (size_t)nscale;
-            if ((st = dalloc(&d_su, cap_sc, s)) || (st = dalloc(&d_sv, cap_sc, s))) {
+            if ((st = dalloc(&d_su, cap_sc, s)) || (st = dalloc(&d_sv, cap_sc, s)) || (st = dalloc(&d_tn, 3 * cap_sc, s))) {
                 free_batch();
                 return st;
             }
@@ -766,45 +1036,55 @@ hmg_status run_aca(hmg_matrix* h, int k, double eps, int precision)
         HMG_CUDA_TRY(cudaMemcpyAsync(d_uo, uo.data(), sizeof(long long) * ne, cudaMemcpyHostToDevice, s));
         HMG_CUDA_TRY(cudaMemcpyAsync(d_vo, vo.data(), sizeof(long long) * ne, cudaMemcpyHostToDevice, s));
         if (mixed) HMG_CUDA_TRY(cudaMemcpyAsync(d_so, so.data(), sizeof(long long) * ne, cudaMemcpyHostToDevice, s));
-        AcaBatch B{d_idx, d_uo, d_vo, dU, dV, d_rank, d_s2};
+        AcaBatch B{d_idx, d_uo, d_vo, dU, dV, d_rank, d_s2, mixed ? d_so : nullptr, mixed ? d_tn : nullptr};
         TierOut T{d_r32, d_r16, d_so, d_su, d_sv};
-        size_t dyn = eps > 0.0 ? (size_t)((maxm1 + 31) / 32) * 4 : 0;
-        if (dyn > 200 * 1024) {
+        const size_t mask = eps > 0.0 ? ((size_t)((maxm1 + 31) / 32) * 4 + 7) & ~(size_t)7 : 0;
+        if (mask > 200 * 1024) {
             set_error("block with %d rows exceeds the adaptive ACA's row-mask capacity", maxm1);
             free_batch();
             return HMG_ERR_UNSUPPORTED;
         }
-        if (dyn > 48 * 1024)
-            HMG_CUDA_TRY(cudaFuncSetAttribute(k_aca, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)dyn));
-        if (eps > 0.0) {
-            // adaptive mode: small blocks one warp each, the others one CTA each
-            std::vector<int> small, large;
-            for (int e = 0; e < ne; e++) {
-                const int bb = idx[e];
-                ((h->h_m1[bb] <= ACA_WSMALL && h->h_m2[bb] <= ACA_WSMALL) ? small : large).push_back(e);
-            }
-            if (!small.empty())
-                HMG_CUDA_TRY(cudaMemcpyAsync(d_list, small.data(), sizeof(int) * small.size(), cudaMemcpyHostToDevice, s));
-            if (!large.empty())
-                HMG_CUDA_TRY(cudaMemcpyAsync(d_list + small.size(), large.data(), sizeof(int) * large.size(),
-                                             cudaMemcpyHostToDevice, s));
-            if (!small.empty()) {
-                const int ns = (int)small.size();
-                k_aca_warp<<<ceil_div(ns, ACA_WPC), ACA_WPC * 32, 0, s>>>(g, h->kspec, P, B, k, eps, d_list, ns);
-                HMG_LAUNCH_CHECK();
-            }
-            if (!large.empty()) {
-                k_aca<<<(unsigned)large.size(), ACA_THREADS, dyn, s>>>(g, h->kspec, P, B, k, eps, d_list + small.size());
-                HMG_LAUNCH_CHECK();
-            }
-            HMG_CUDA_TRY(cudaStreamSynchronize(s));  // the host vectors go out of scope
-        } else {
-            k_aca<<<ne, ACA_THREADS, dyn, s>>>(g, h->kspec, P, B, k, eps, nullptr);
-            HMG_LAUNCH_CHECK();
+        // the blocks by class, in each the ones with most work first
+        std::vector<int> list(ne);
+        std::vector<int> cls(ne);
+        int count[ACA_NCLASS] = {}, first[ACA_NCLASS], at[ACA_NCLASS];
+        for (int e = 0; e < ne; e++) {
+            const int side = std::max(h->h_m1[idx[e]], h->h_m2[idx[e]]);
+            int c = 0;
+            while (side > ACA_CLASSES[c].side) c++;
+            cls[e] = c;
+            count[c]++;
+        }
+        for (int c = ACA_NCLASS - 1, o = 0; c >= 0; o += count[c], c--) first[c] = at[c] = o;
+        for (int e = 0; e < ne; e++) list[at[cls[e]]++] = e;
+        std::stable_sort(list.begin(), list.begin() + count[ACA_NCLASS - 1], [&](int x, int y) {
+            return (long long)h->h_m1[idx[x]] + h->h_m2[idx[x]] > (long long)h->h_m1[idx[y]] + h->h_m2[idx[y]];
+        });
+        HMG_CUDA_TRY(cudaMemcpyAsync(d_list, list.data(), sizeof(int) * ne, cudaMemcpyHostToDevice, s));
+        // on three streams, so that one class's last blocks overlap the next class's first ones
+        if ((st = ensure_side_streams(h))) {
+            free_batch();
+            return st;
+        }
+        HMG_CUDA_TRY(cudaEventRecord(h->k1_ev[0], s));
+        for (int i = 0; i < 2; i++) HMG_CUDA_TRY(cudaStreamWaitEvent(h->k1_aux[i], h->k1_ev[0], 0));
+        auto kc = [&](int c) { return (std::min(k, ACA_CLASSES[c].side) + 1) & ~1; };
+        auto bits = [&](int c) { return eps <= 0.0 ? 0 : (c < ACA_NCLASS - 1 ? ACA_CLASSES[c].side / 8 : (int)mask); };
+        const int big = std::max(0, ACA_CLASSES[3].panel - bits(3)) & ~15;
+        if ((st = launch_aca<512, 2, 1>(g, h->kspec, P, B, k, eps, d_list + first[3], count[3], big, kc(3), bits(3), s)) ||
+            (st = launch_aca<512, 1, 2>(g, h->kspec, P, B, k, eps, d_list + first[2], count[2], ACA_CLASSES[2].panel, kc(2), bits(2), h->k1_aux[0])) ||
+            (st = launch_aca<256, 1, 3>(g, h->kspec, P, B, k, eps, d_list + first[1], count[1], ACA_CLASSES[1].panel, kc(1), bits(1), h->k1_aux[1])) ||
+            (st = launch_small(g, h->kspec, P, B, k, eps, d_list + first[0], count[0], kc(0), bits(0), h->k1_aux[0]))) {
+            cudaDeviceSynchronize();
+            free_batch();
+            return st;
+        }
+        for (int i = 0; i < 2; i++) {
+            HMG_CUDA_TRY(cudaEventRecord(h->k1_ev[1 + i], h->k1_aux[i]));
+            HMG_CUDA_TRY(cudaStreamWaitEvent(s, h->k1_ev[1 + i], 0));
         }
         if (mixed) {
-            k_aca_tiers<<<ne, 256, 0, s>>>(g, B, T);
+            k_aca_tiers<<<ceil_div(ne, 8), 256, 0, s>>>(B, T, ne);
             HMG_LAUNCH_CHECK();
         }
         std::vector<int> br(ne), b32(ne, 0), b16(ne, 0);

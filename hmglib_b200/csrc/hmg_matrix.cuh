@@ -144,7 +144,7 @@ struct hmg_matrix {
     int k1_grid = 0, k2_grid = 0;
     bool profiling = false;
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
-    cudaStream_t k1_aux[2] = {nullptr, nullptr};  // side streams of the FP16 / FP8 V^T x tiers (matvec.cu)
+    cudaStream_t k1_aux[2] = {nullptr, nullptr};  // side streams: FP16 / FP8 V^T x tiers (matvec.cu), ACA classes (aca.cu)
     cudaEvent_t k1_ev[3] = {nullptr, nullptr, nullptr};  // their fork and joins
 };
 
@@ -160,6 +160,7 @@ hmg_status save(hmg_matrix* h, const char* path);
 hmg_status load(hmg_matrix** out, const char* path, cudaStream_t s);
 hmg_status run_aca(hmg_matrix* h, int k, double eps, int precision);
 hmg_status fill_near(hmg_matrix* h, int precision);
+hmg_status ensure_side_streams(hmg_matrix* h);
 hmg_status matvec_device(hmg_matrix* h, const double* x, double* y, bool fp64_arith = false);
 hmg_status matvec_unbatched(hmg_matrix* h, const double* x, double* y);
 hmg_status matvec_multi(hmg_matrix* h, int nrhs, const double* X, int ldx, double* Y, int ldy);

@@ -832,6 +832,17 @@ static hmg_status launch_product_graph(hmg_matrix* h, const double* x, double* y
     return HMG_OK;
 }
 
+// The handle's two side streams and the events that fork them from and join them into
+// its stream.
+hmg_status ensure_side_streams(hmg_matrix* h)
+{
+    for (int i = 0; i < 2; i++)
+        if (!h->k1_aux[i]) HMG_CUDA_TRY(cudaStreamCreateWithFlags(&h->k1_aux[i], cudaStreamNonBlocking));
+    for (int i = 0; i < 3; i++)
+        if (!h->k1_ev[i]) HMG_CUDA_TRY(cudaEventCreateWithFlags(&h->k1_ev[i], cudaEventDisableTiming));
+    return HMG_OK;
+}
+
 // The launches of one product (x gather, V^T x per storage tier, tile kernel).
 static hmg_status launch_product(hmg_matrix* h, const double* x, double* y, bool fp64, bool arith64, bool bulk_k1,
                                  bool bulk_k2)
@@ -855,10 +866,7 @@ static hmg_status launch_product(hmg_matrix* h, const double* x, double* y, bool
         // tier's load-bound ones and the three launches' tails overlap.
         const bool fork = h->k1_task_start[1][4] > 0 || h->k1_task_start[2][4] > 0;
         if (fork) {
-            for (int i = 0; i < 2; i++)
-                if (!h->k1_aux[i]) HMG_CUDA_TRY(cudaStreamCreateWithFlags(&h->k1_aux[i], cudaStreamNonBlocking));
-            for (int i = 0; i < 3; i++)
-                if (!h->k1_ev[i]) HMG_CUDA_TRY(cudaEventCreateWithFlags(&h->k1_ev[i], cudaEventDisableTiming));
+            if ((st = ensure_side_streams(h))) return st;
             HMG_CUDA_TRY(cudaEventRecord(h->k1_ev[0], s));
             for (int i = 0; i < 2; i++) HMG_CUDA_TRY(cudaStreamWaitEvent(h->k1_aux[i], h->k1_ev[0], 0));
         }
