@@ -119,6 +119,11 @@ struct hmg_matrix {
     float* xs32 = nullptr;
     void* tbuf = nullptr;     // V^T x per block (rank_total entries)
     void* pair_desc = nullptr;     // per (tile, block) pair: slice pointer, vector, columns
+    // what the tile kernels walk: the pairs, those of more than TILE_CHUNK columns cut into
+    // runs of that many (both arrays are the ones above where no pair is that long)
+    void* tile_desc = nullptr;
+    int* tile_desc_start = nullptr;
+    bool tile_desc_own = false;
     int desc_near_mode = -1, desc_near_prec = -2, desc_far_prec = -2, desc_elem = 0;
     void* k1_units = nullptr;      // K1 pieces of V^T (rows of one storage tier), grouped by tier
     int nk1 = 0;

@@ -217,6 +217,95 @@ __global__ void k_build_k1desc(const K1Unit* units, int n, const int* blk_c0, co
 // loads in flight whatever the tier.
 static constexpr int k1_nch(int tier) { return tier == 0 ? 2 : (tier == 1 ? 4 : 8); }
 
+// Long dense pairs.  Where points cluster, Z-order cells of one level differ a thousandfold
+// in size, and a leaf's tile meets dense blocks of tens of thousands of columns: one warp
+// walked such a pair alone while the rest of the GPU was idle (131072 clustered points in
+// 2D, FP32: 1.74 ms in the tile kernel, against 0.2 ms of it with more than one SM at
+// work).  Pairs of more than TILE_CHUNK columns are cut into runs of that many, which the
+// CTA's warps share; 256 columns are two to four times an ordinary dense pair, so that the
+// lists of evenly spread points stay as they are.
+__global__ void k_count_chunks(const PairDesc* desc, const int* start, int ntiles, int* count)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t > ntiles) return;
+    int n = 0;
+    if (t < ntiles)
+        for (int p = start[t]; p < start[t + 1]; p++) {
+            const bool dense = desc[p].kind == PAIR_STORED || desc[p].kind == PAIR_ONTHEFLY;
+            n += dense ? max(1, (desc[p].ncol + TILE_CHUNK - 1) / TILE_CHUNK) : 1;
+        }
+    count[t] = n;
+}
+
+// (w_elem: bytes of a vector element; near_esz: of a stored entry)
+__global__ void k_write_chunks(const PairDesc* desc, const int* start, int ntiles, const int* tile_s, const int* chunk_start,
+                               int w_elem, int near_esz, PairDesc* out)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= ntiles) return;
+    const size_t col = (size_t)((tile_s[t] + 3) & ~3) * near_esz;
+    int o = chunk_start[t];
+    for (int p = start[t]; p < start[t + 1]; p++) {
+        const PairDesc d = desc[p];
+        const bool dense = d.kind == PAIR_STORED || d.kind == PAIR_ONTHEFLY;
+        if (!dense || d.ncol <= TILE_CHUNK) {
+            out[o++] = d;
+            continue;
+        }
+        for (int j = 0; j < d.ncol; j += TILE_CHUNK) {
+            PairDesc c = d;
+            c.ncol = min(TILE_CHUNK, d.ncol - j);
+            c.c0 = d.c0 + j;
+            c.w = static_cast<const char*>(d.w) + (size_t)j * w_elem;
+            if (d.data) c.data = static_cast<const char*>(d.data) + (size_t)j * col;
+            out[o++] = c;
+        }
+    }
+}
+
+void free_tile_desc(hmg_matrix* h)
+{
+    if (h->tile_desc_own) {
+        dfree(h->tile_desc, h->stream);
+        dfree(h->tile_desc_start, h->stream);
+    }
+    h->tile_desc = nullptr;
+    h->tile_desc_start = nullptr;
+    h->tile_desc_own = false;
+}
+
+static hmg_status build_tile_desc(hmg_matrix* h, int elem, int near_esz)
+{
+    cudaStream_t s = h->stream;
+    free_tile_desc(h);
+    int longest = 0;
+    for (int b = 0; b < h->ndense; b++) longest = std::max(longest, h->h_m2[b]);
+    if (longest <= TILE_CHUNK || h->ntiles <= 0) {
+        h->tile_desc = h->pair_desc;
+        h->tile_desc_start = h->tile_pair_start;
+        return HMG_OK;
+    }
+    hmg_status st;
+    const int nt = h->ntiles;
+    const PairDesc* pd = static_cast<const PairDesc*>(h->pair_desc);
+    int* start = nullptr;
+    if ((st = dalloc(&start, (size_t)nt + 1, s))) return st;
+    h->tile_desc_start = start;
+    h->tile_desc_own = true;
+    k_count_chunks<<<ceil_div(nt + 1, 128), 128, 0, s>>>(pd, h->tile_pair_start, nt, start);
+    HMG_LAUNCH_CHECK();
+    if ((st = scan_exclusive<int>(start, start, nt + 1, nullptr, s))) return st;
+    int total = 0;
+    HMG_CUDA_TRY(cudaMemcpyAsync(&total, start + nt, sizeof(int), cudaMemcpyDeviceToHost, s));
+    HMG_CUDA_TRY(cudaStreamSynchronize(s));
+    PairDesc* out = nullptr;
+    if ((st = dalloc(&out, (size_t)(total > 0 ? total : 1), s))) return st;
+    h->tile_desc = out;
+    k_write_chunks<<<ceil_div(nt, 128), 128, 0, s>>>(pd, h->tile_pair_start, nt, h->tile_s, start, elem, near_esz, out);
+    HMG_LAUNCH_CHECK();
+    return HMG_OK;
+}
+
 hmg_status ensure_desc(hmg_matrix* h, int elem)
 {
     cudaStream_t s = h->stream;
@@ -243,6 +332,7 @@ hmg_status ensure_desc(hmg_matrix* h, int elem)
             h->far_prec == HMG_PREC_MIXED ? 1 : 0, (PairDesc*)h->pair_desc);
         HMG_LAUNCH_CHECK();
     }
+    if ((st = build_tile_desc(h, elem, near_esz))) return st;
     // K1 pieces: terms of V_b^T of one storage tier, in runs of at most k1_piece_bytes
     // (64 KB unless hmg_autotune chose otherwise).  Each
     // piece gets the widest lane group 2^LG (LG 2..5) whose lanes still get k1_nch
@@ -767,10 +857,10 @@ static ProductKey product_key(hmg_matrix* h, const double* x, double* y, bool fp
     memcpy(k.k1_piece_start, h->k1_piece_start, sizeof(k.k1_piece_start));
     k.k1_units = h->k1_units;
     k.tbuf = h->tbuf;
-    k.pair_desc = h->pair_desc;
+    k.pair_desc = h->tile_desc;
     k.xs64 = h->xs64;
     k.xs32 = h->xs32;
-    k.tile_pair_start = h->tile_pair_start;
+    k.tile_pair_start = h->tile_desc_start;
     k.tile_r0 = h->tile_r0;
     k.tile_s = h->tile_s;
     k.perm0 = h->perm[0];
@@ -910,15 +1000,15 @@ static hmg_status launch_product(hmg_matrix* h, const double* x, double* y, bool
     if (h->ntiles > 0 && bulk_k2) {
         if ((st = launch_tiles_bulk(h, fp64, y))) return st;
     } else if (h->ntiles > 0) {
-        const PairDesc* pd = static_cast<const PairDesc*>(h->pair_desc);
+        const PairDesc* pd = static_cast<const PairDesc*>(h->tile_desc);
         if (fp64)
-            k_tile_matvec<double, double><<<h->ntiles, 256, 0, s>>>(pd, h->tile_pair_start, h->tile_r0, h->tile_s,
+            k_tile_matvec<double, double><<<h->ntiles, 256, 0, s>>>(pd, h->tile_desc_start, h->tile_r0, h->tile_s,
                                                                     h->perm[0], h->kspec, P, h->xs64, y);
         else if (arith64)
-            k_tile_matvec<float, double><<<h->ntiles, 256, 0, s>>>(pd, h->tile_pair_start, h->tile_r0, h->tile_s,
+            k_tile_matvec<float, double><<<h->ntiles, 256, 0, s>>>(pd, h->tile_desc_start, h->tile_r0, h->tile_s,
                                                                    h->perm[0], h->kspec, P, h->xs64, y);
         else
-            k_tile_matvec<float, float><<<h->ntiles, 256, 0, s>>>(pd, h->tile_pair_start, h->tile_r0, h->tile_s,
+            k_tile_matvec<float, float><<<h->ntiles, 256, 0, s>>>(pd, h->tile_desc_start, h->tile_r0, h->tile_s,
                                                                   h->perm[0], h->kspec, P, h->xs64, y);
         HMG_LAUNCH_CHECK();
     }

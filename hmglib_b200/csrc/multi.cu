@@ -162,7 +162,7 @@ static hmg_status launch_multi(hmg_matrix* h, int nrhs, const double* X, int ldx
         HMG_LAUNCH_CHECK();
     }
     if (h->ntiles > 0) {
-        k_tile_multi<R><<<h->ntiles, 256, 0, s>>>(static_cast<const PairDesc*>(h->pair_desc), h->tile_pair_start,
+        k_tile_multi<R><<<h->ntiles, 256, 0, s>>>(static_cast<const PairDesc*>(h->tile_desc), h->tile_desc_start,
                                                   h->tile_r0, h->tile_s, h->perm[0], xm, tm,
                                                   static_cast<const char*>(h->tbuf), nrhs, Y, ldy);
         HMG_LAUNCH_CHECK();

@@ -835,7 +835,7 @@ static hmg_status launch_tiles(hmg_matrix* h, const float* xm, const float* tm, 
     if (h->ntiles <= 0) return HMG_OK;
     HMG_CUDA_TRY(cudaFuncSetAttribute(k_tile_tf32<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, TtShape<NT>::SMEM));
     k_tile_tf32<NT><<<h->ntiles, TtShape<NT>::WARPS * 32, TtShape<NT>::SMEM, h->stream>>>(
-        static_cast<const PairDesc*>(h->pair_desc), h->tile_pair_start, h->tile_r0, h->tile_s, h->perm[0], xm, tm,
+        static_cast<const PairDesc*>(h->tile_desc), h->tile_desc_start, h->tile_r0, h->tile_s, h->perm[0], xm, tm,
         static_cast<const char*>(h->tbuf), nrhs, Y, ldy, only_kind, wide);
     HMG_LAUNCH_CHECK();
     return HMG_OK;

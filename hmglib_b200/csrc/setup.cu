@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "hmg_matrix.cuh"
+#include "stream.cuh"
 
 namespace hmg {
 
@@ -409,6 +410,8 @@ void free_tree(hmg_matrix* h)
     dfree(h->blk_type, s);
     dfree(h->tile_r0, s); dfree(h->tile_s, s); dfree(h->tile_pstart, s);
     dfree(h->blk_tfirst, s); dfree(h->blk_tlast, s);
+    free_tile_desc(h);
+    dfree(h->pair_desc, s);  // sized for this tree's pairs
     dfree(h->tile_pair_start, s); dfree(h->pair_block, s);
     dfree(h->blk_param, s);
     h->nblocks = h->ndense = h->naca = h->ntiles = h->npairs = h->levels = 0;

@@ -48,12 +48,15 @@ __device__ __forceinline__ uint4 ld_stream(const void* p)
         : "l"(p));
     return v;
 }
+// longest pair a tile kernel's warp takes whole (see free_tile_desc)
+static constexpr int TILE_CHUNK = 256;
 // largest rank the streaming V^T x kernel accepts
 static constexpr int K1_MAXRANK = 128;
 
 hmg_status launch_tiles_bulk(hmg_matrix* h, bool fp64, double* y);
 // pair and K1 descriptors for products in arithmetic of elem bytes (matvec.cu)
 hmg_status ensure_desc(hmg_matrix* h, int elem);
+void free_tile_desc(hmg_matrix* h);
 // padded, zeroed Z-ordered x buffers (matvec.cu)
 hmg_status ensure_xs(hmg_matrix* h);
 hmg_status launch_vtx_bulk(hmg_matrix* h, bool fp64);
