@@ -222,19 +222,44 @@ struct AcaBlock {
                 val[q] = __fma_rn(-coef[l], *sq[q], val[q]);
                 sq[q] += ms;
             }
+        // (l = cap, a multiple of 4, where there are terms in the scratch)
         if (AHEAD) {
-            for (; l < r; l += 8, g += 8 * (size_t)ld) {
+            const double* p[N];  // the next term to load
 #pragma unroll
-                for (int u = 0; u < 8; u++) {
-                    if (l + u >= r) break;
-                    const double c = coef[l + u];
+            for (int q = 0; q < N; q++) p[q] = g + 8 * (size_t)ld + idx[q];
+            for (; l + 16 <= r; l += 8) {
 #pragma unroll
-                    for (int q = 0; q < N; q++) val[q] = __fma_rn(-c, t[u][q], val[q]);
-                    if (l + u + 8 < r)
+                for (int u = 0; u < 8; u += 2) {
+                    const double2 c = *reinterpret_cast<const double2*>(coef + l + u);
 #pragma unroll
-                        for (int q = 0; q < N; q++) t[u][q] = __ldcg(g + (size_t)(u + 8) * ld + idx[q]);
+                    for (int q = 0; q < N; q++) {
+                        val[q] = __fma_rn(-c.x, t[u][q], val[q]);
+                        t[u][q] = __ldcg(p[q]);
+                        p[q] += ld;
+                        val[q] = __fma_rn(-c.y, t[u + 1][q], val[q]);
+                        t[u + 1][q] = __ldcg(p[q]);
+                        p[q] += ld;
+                    }
                 }
             }
+            const int have = min(8, r - l);  // loaded; then the rest, fewer than 8
+#pragma unroll
+            for (int u = 0; u < 8; u++)
+                if (u < have) {
+                    const double c = coef[l + u];
+#pragma unroll
+                    for (int q = 0; q < N; q++) {
+                        val[q] = __fma_rn(-c, t[u][q], val[q]);
+                        if (l + u + 8 < r) t[u][q] = __ldcg(p[q] + (size_t)u * ld);
+                    }
+                }
+#pragma unroll
+            for (int u = 0; u < 8; u++)
+                if (l + u + 8 < r) {
+                    const double c = coef[l + u + 8];
+#pragma unroll
+                    for (int q = 0; q < N; q++) val[q] = __fma_rn(-c, t[u][q], val[q]);
+                }
         } else {
             for (; l + 8 <= r; l += 8, g += 8 * (size_t)ld) {
 #pragma unroll
@@ -242,9 +267,14 @@ struct AcaBlock {
 #pragma unroll
                     for (int q = 0; q < N; q++) t[u][q] = __ldcg(g + (size_t)u * ld + idx[q]);
 #pragma unroll
-                for (int u = 0; u < 8; u++)
+                for (int u = 0; u < 8; u += 2) {
+                    const double2 c = *reinterpret_cast<const double2*>(coef + l + u);
 #pragma unroll
-                    for (int q = 0; q < N; q++) val[q] = __fma_rn(-coef[l + u], t[u][q], val[q]);
+                    for (int q = 0; q < N; q++) {
+                        val[q] = __fma_rn(-c.x, t[u][q], val[q]);
+                        val[q] = __fma_rn(-c.y, t[u + 1][q], val[q]);
+                    }
+                }
             }
             for (; l < r; l++, g += ld)
 #pragma unroll
@@ -369,7 +399,7 @@ k_aca(BlockGeom g, KernelSpec K0, PointsView P, AcaBatch B, int k, double eps, c
     kb = kb < m2 ? kb : m2;
     const int tid = threadIdx.x;
     unsigned* used = reinterpret_cast<unsigned*>(coef2 + kc);
-    const AcaBlock<T, C> A{sh, aca_smem, m1 + m2, panel / (m1 + m2), B.U + B.uoff[e], B.V + B.voff[e], m1, m2,
+    const AcaBlock<T, C> A{sh, aca_smem, m1 + m2, panel / (m1 + m2) & ~3, B.U + B.uoff[e], B.V + B.voff[e], m1, m2,
                         tid, tid & 31, tid >> 5};
     const bool adaptive = eps > 0.0;
     int rank = 0;
@@ -938,38 +968,38 @@ hmg_status run_aca(hmg_matrix* h, int k, double eps, int precision)
 
     // Scratch of the batches, grown to the largest batch and reused across batches.  The
     // factors' part is up to 4 GB, which the stream-ordered pool maps and unmaps at 6.3 ms a
-    // GB each way, cudaMalloc and cudaFree at 0.2 and 0.6 (measured): beyond what the pool
-    // keeps it comes from cudaMalloc.
-    static constexpr size_t POOL_SCRATCH = POOL_KEEP / 8 / sizeof(double);
+    // GB each way; a cudaMalloc and its cudaFree take 0.7 ms and 0.8 more a GB (measured), so
+    // from 64 MB on it comes from there.
+    static constexpr size_t POOL_SCRATCH = (64u << 20) / sizeof(double);
     int* d_idx = nullptr;
     long long *d_uo = nullptr, *d_vo = nullptr, *d_so = nullptr;
-    double *dU = nullptr, *dV = nullptr, *d_s2 = nullptr, *d_tn = nullptr;
+    double *dU = nullptr, *d_s2 = nullptr, *d_tn = nullptr;  // dU: the batch's u terms, then its v terms
     int *d_rank = nullptr, *d_r32 = nullptr, *d_r16 = nullptr, *d_list = nullptr;
     float *d_su = nullptr, *d_sv = nullptr;
-    size_t cap_ne = 0, cap_u = 0, cap_v = 0, cap_sc = 0;
-    auto drop = [&](double*& p, size_t cap) {
-        if (cap <= POOL_SCRATCH) dfree(p, s);
-        else if (p) cudaFree(p);
-        p = nullptr;
+    size_t cap_ne = 0, cap_uv = 0, cap_sc = 0;
+    auto drop = [&]() {
+        if (cap_uv <= POOL_SCRATCH) dfree(dU, s);
+        else if (dU) cudaFree(dU);
+        dU = nullptr;
+        cap_uv = 0;
     };
-    auto grow = [&](double*& p, size_t& cap, size_t n) {
-        drop(p, cap);
-        cap = n > 0 ? n : 1;
-        if (cap <= POOL_SCRATCH) return dalloc(&p, cap, s);
-        const cudaError_t e = cudaMalloc((void**)&p, cap * sizeof(double));
+    auto grow = [&](size_t n) {
+        drop();
+        cap_uv = n > 0 ? n : 1;
+        if (cap_uv <= POOL_SCRATCH) return dalloc(&dU, cap_uv, s);
+        const cudaError_t e = cudaMalloc((void**)&dU, cap_uv * sizeof(double));
         if (e == cudaSuccess) return HMG_OK;
         cudaGetLastError();
-        p = nullptr;
-        set_error("allocating %zu bytes of ACA scratch failed: %s", cap * sizeof(double), cudaGetErrorString(e));
+        dU = nullptr;
+        set_error("allocating %zu bytes of ACA scratch failed: %s", cap_uv * sizeof(double), cudaGetErrorString(e));
         return e == cudaErrorMemoryAllocation ? HMG_ERR_NOMEM : HMG_ERR_CUDA;
     };
     auto free_batch = [&]() {
-        drop(dU, cap_u);
-        drop(dV, cap_v);
+        drop();
         dfree(d_idx, s); dfree(d_uo, s); dfree(d_vo, s);
         dfree(d_rank, s); dfree(d_s2, s); dfree(d_so, s); dfree(d_r32, s); dfree(d_r16, s);
         dfree(d_su, s); dfree(d_sv, s); dfree(d_tn, s); dfree(d_list, s);
-        cap_ne = cap_u = cap_v = cap_sc = 0;
+        cap_ne = cap_sc = 0;
     };
     int bstart = h->ndense;
     while (bstart < nb) {
@@ -1010,17 +1040,9 @@ hmg_status run_aca(hmg_matrix* h, int k, double eps, int precision)
                 return st;
             }
         }
-        if ((size_t)us > cap_u) {
-            if ((st = grow(dU, cap_u, (size_t)us))) {
-                free_batch();
-                return st;
-            }
-        }
-        if ((size_t)vs > cap_v) {
-            if ((st = grow(dV, cap_v, (size_t)vs))) {
-                free_batch();
-                return st;
-            }
+        if ((size_t)(us + vs) > cap_uv && (st = grow((size_t)(us + vs)))) {
+            free_batch();
+            return st;
         }
         if (mixed && (size_t)nscale > cap_sc) {
             dfree(d_su, s);
@@ -1036,7 +1058,7 @@ hmg_status run_aca(hmg_matrix* h, int k, double eps, int precision)
         HMG_CUDA_TRY(cudaMemcpyAsync(d_uo, uo.data(), sizeof(long long) * ne, cudaMemcpyHostToDevice, s));
         HMG_CUDA_TRY(cudaMemcpyAsync(d_vo, vo.data(), sizeof(long long) * ne, cudaMemcpyHostToDevice, s));
         if (mixed) HMG_CUDA_TRY(cudaMemcpyAsync(d_so, so.data(), sizeof(long long) * ne, cudaMemcpyHostToDevice, s));
-        AcaBatch B{d_idx, d_uo, d_vo, dU, dV, d_rank, d_s2, mixed ? d_so : nullptr, mixed ? d_tn : nullptr};
+        AcaBatch B{d_idx, d_uo, d_vo, dU, dU + us, d_rank, d_s2, mixed ? d_so : nullptr, mixed ? d_tn : nullptr};
         TierOut T{d_r32, d_r16, d_so, d_su, d_sv};
         const size_t mask = eps > 0.0 ? ((size_t)((maxm1 + 31) / 32) * 4 + 7) & ~(size_t)7 : 0;
         if (mask > 200 * 1024) {
@@ -1061,25 +1083,33 @@ hmg_status run_aca(hmg_matrix* h, int k, double eps, int precision)
             return (long long)h->h_m1[idx[x]] + h->h_m2[idx[x]] > (long long)h->h_m1[idx[y]] + h->h_m2[idx[y]];
         });
         HMG_CUDA_TRY(cudaMemcpyAsync(d_list, list.data(), sizeof(int) * ne, cudaMemcpyHostToDevice, s));
-        // on three streams, so that one class's last blocks overlap the next class's first ones
-        if ((st = ensure_side_streams(h))) {
-            free_batch();
-            return st;
+        // on three streams, so that one class's last blocks overlap the next class's first
+        // ones; a small batch (the streams and events of a new handle take 0.25 ms to make and
+        // destroy, 1700 points at rank 32 3.5 ms to build and multiply) stays on the handle's
+        const bool fork = us + vs > (16ll << 20);
+        cudaStream_t on[ACA_NCLASS] = {s, s, s, s};
+        if (fork) {
+            if ((st = ensure_side_streams(h))) {
+                free_batch();
+                return st;
+            }
+            HMG_CUDA_TRY(cudaEventRecord(h->k1_ev[0], s));
+            for (int i = 0; i < 2; i++) HMG_CUDA_TRY(cudaStreamWaitEvent(h->k1_aux[i], h->k1_ev[0], 0));
+            on[0] = on[2] = h->k1_aux[0];
+            on[1] = h->k1_aux[1];
         }
-        HMG_CUDA_TRY(cudaEventRecord(h->k1_ev[0], s));
-        for (int i = 0; i < 2; i++) HMG_CUDA_TRY(cudaStreamWaitEvent(h->k1_aux[i], h->k1_ev[0], 0));
         auto kc = [&](int c) { return (std::min(k, ACA_CLASSES[c].side) + 1) & ~1; };
         auto bits = [&](int c) { return eps <= 0.0 ? 0 : (c < ACA_NCLASS - 1 ? ACA_CLASSES[c].side / 8 : (int)mask); };
         const int big = std::max(0, ACA_CLASSES[3].panel - bits(3)) & ~15;
         if ((st = launch_aca<512, 2, 1>(g, h->kspec, P, B, k, eps, d_list + first[3], count[3], big, kc(3), bits(3), s)) ||
-            (st = launch_aca<512, 1, 2>(g, h->kspec, P, B, k, eps, d_list + first[2], count[2], ACA_CLASSES[2].panel, kc(2), bits(2), h->k1_aux[0])) ||
-            (st = launch_aca<256, 1, 3>(g, h->kspec, P, B, k, eps, d_list + first[1], count[1], ACA_CLASSES[1].panel, kc(1), bits(1), h->k1_aux[1])) ||
-            (st = launch_small(g, h->kspec, P, B, k, eps, d_list + first[0], count[0], kc(0), bits(0), h->k1_aux[0]))) {
+            (st = launch_aca<512, 1, 2>(g, h->kspec, P, B, k, eps, d_list + first[2], count[2], ACA_CLASSES[2].panel, kc(2), bits(2), on[2])) ||
+            (st = launch_aca<256, 1, 3>(g, h->kspec, P, B, k, eps, d_list + first[1], count[1], ACA_CLASSES[1].panel, kc(1), bits(1), on[1])) ||
+            (st = launch_small(g, h->kspec, P, B, k, eps, d_list + first[0], count[0], kc(0), bits(0), on[0]))) {
             cudaDeviceSynchronize();
             free_batch();
             return st;
         }
-        for (int i = 0; i < 2; i++) {
+        for (int i = 0; i < 2 && fork; i++) {
             HMG_CUDA_TRY(cudaEventRecord(h->k1_ev[1 + i], h->k1_aux[i]));
             HMG_CUDA_TRY(cudaStreamWaitEvent(s, h->k1_ev[1 + i], 0));
         }
