@@ -58,14 +58,17 @@ __global__ void k_mr_dot_partial(const double* a, long long lda, const double* b
     }
 }
 
-// out[j] = sum of column j's partials, in order
+// out[j] = sum of column j's partials, a warp a column: lane l adds partials l, l + 32, ...
+// in order and a butterfly adds the lanes (one thread a column waited for 148 dependent
+// additions: 11.6 us against 2.5 us, twice an iteration)
 __global__ void k_mr_dot_final(const double* part, int np, int k, double* out)
 {
-    const int j = threadIdx.x;
-    if (j >= k) return;
+    const int j = blockIdx.x, lane = threadIdx.x;
     double s = 0.0;
-    for (int i = 0; i < np; i++) s += part[(size_t)j * np + i];
-    out[j] = s;
+    for (int i = lane; i < np; i += 32) s += part[(size_t)j * np + i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0 && j < k) out[j] = s;
 }
 
 // Column scalars of the recurrence, one thread per column.
@@ -225,7 +228,7 @@ static hmg_status mr_dot(hmg_cg_multi* c, const double* a, const double* b, doub
     cudaStream_t st = c->h->stream;
     k_mr_dot_partial<<<dim3(MR_BLOCKS, c->k), MR_THREADS, 0, st>>>(a, c->n, b, c->n, c->n, c->part);
     HMG_LAUNCH_CHECK();
-    k_mr_dot_final<<<1, 64, 0, st>>>(c->part, MR_BLOCKS, c->k, out);
+    k_mr_dot_final<<<c->k, 32, 0, st>>>(c->part, MR_BLOCKS, c->k, out);
     HMG_LAUNCH_CHECK();
     return HMG_OK;
 }
