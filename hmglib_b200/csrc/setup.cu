@@ -191,45 +191,65 @@ __device__ int split_index(const uint64_t* codes, int first, int last)
 // One CTA per cluster [l,u]: exact bounding box into the per-level maps (indexed by
 // l), and the split point for clusters that may be subdivided.  leaf_at (grouped
 // point sets, else null) gives the leaf size of the set that holds each point.
-__global__ void k_cluster_bbox(const int* cl_l, const int* cl_u, int ncl, const double* z,
-                               int n, int dim, const uint64_t* codes, int c_leaf, const int* leaf_at,
-                               double* bb_lo, double* bb_hi, int* split_of)
+// Bound by the latency of the first levels' loads, whose few CTAs read all points: up to
+// 1024 threads, four points of every dimension in flight each (all levels of both sides:
+// N = 131071 in 3D 3.07 ms with 256 threads and one load, 0.57 now; 16384 in 2D 0.41, 0.22).
+static constexpr int BBOX_MAX_THREADS = 1024;
+__global__ void __launch_bounds__(BBOX_MAX_THREADS)
+k_cluster_bbox(const int* cl_l, const int* cl_u, int ncl, const double* z,
+               int n, int dim, const uint64_t* codes, int c_leaf, const int* leaf_at,
+               double* bb_lo, double* bb_hi, int* split_of)
 {
-    __shared__ double red[2][3][8];
+    __shared__ double red[2][3][BBOX_MAX_THREADS / 32];
     int c = blockIdx.x;
     if (c >= ncl) return;
     int l = cl_l[c], u = cl_u[c];
     int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int d = 0; d < dim; d++) {
-        const double* zc = z + (size_t)d * n;
-        double lo = zc[l], hi = zc[l];
-        for (int i = l + threadIdx.x; i <= u; i += blockDim.x) {
-            double v = zc[i];
-            lo = fmin(lo, v);
-            hi = fmax(hi, v);
-        }
+    double lo[3], hi[3];
+    for (int d = 0; d < dim; d++) lo[d] = hi[d] = z[(size_t)d * n + l];
+    for (int i = l + threadIdx.x; i <= u; i += 4 * blockDim.x) {
+        double v[3][4];
+#pragma unroll
+        for (int d = 0; d < 3; d++)
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if (d < dim) v[d][k] = z[(size_t)d * n + min(i + k * (int)blockDim.x, u)];
+#pragma unroll
+        for (int d = 0; d < 3; d++)
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if (d < dim) {
+                    lo[d] = fmin(lo[d], v[d][k]);
+                    hi[d] = fmax(hi[d], v[d][k]);
+                }
+    }
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        if (d >= dim) break;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
-            lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-            hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+            lo[d] = fmin(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+            hi[d] = fmax(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
         }
         if (lane == 0) {
-            red[0][d][warp] = lo;
-            red[1][d][warp] = hi;
+            red[0][d][warp] = lo[d];
+            red[1][d][warp] = hi[d];
         }
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int nw = blockDim.x >> 5;
-        for (int d = 0; d < dim; d++) {
-            double lo = red[0][d][0], hi = red[1][d][0];
-            for (int w = 1; w < nw; w++) {
-                lo = fmin(lo, red[0][d][w]);
-                hi = fmax(hi, red[1][d][w]);
-            }
-            bb_lo[(size_t)d * n + l] = lo;
-            bb_hi[(size_t)d * n + l] = hi;
+    if (warp < dim) {  // a warp a dimension
+        const int nw = blockDim.x >> 5, w = min(lane, nw - 1);
+        double a = red[0][warp][w], b = red[1][warp][w];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            a = fmin(a, __shfl_xor_sync(0xffffffffu, a, o));
+            b = fmax(b, __shfl_xor_sync(0xffffffffu, b, o));
         }
+        if (lane == 0) {
+            bb_lo[(size_t)warp * n + l] = a;
+            bb_hi[(size_t)warp * n + l] = b;
+        }
+    } else if (warp == 3 && lane == 0) {
         if (u - l + 1 > (leaf_at ? leaf_at[l] : c_leaf)) split_of[l] = split_index(codes, l, u);
     }
 }
@@ -485,7 +505,10 @@ static hmg_status traverse(hmg_matrix* h, int nroots, const int* rl1, const int*
         for (int set = 0; set < 2; set++) {
             ClusterSet& c = cs[set];
             if (c.ncl > 0) {
-                k_cluster_bbox<<<c.ncl, 256, 0, s>>>(c.cl_l, c.cl_u, c.ncl, h->zpts[set], c.n, dim,
+                // threads for the mean cluster: 256 points four at a time a CTA of 128 and up
+                int threads = 128;
+                while (threads < BBOX_MAX_THREADS && (long long)threads * 8 * c.ncl < c.n) threads *= 2;
+                k_cluster_bbox<<<c.ncl, threads, 0, s>>>(c.cl_l, c.cl_u, c.ncl, h->zpts[set], c.n, dim,
                                                      h->codes[set], h->c_leaf, leaf_at[set], c.bb_lo,
                                                      c.bb_hi, c.split_of);
                 HMG_LAUNCH_CHECK();
