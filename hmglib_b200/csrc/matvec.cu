@@ -321,6 +321,7 @@ hmg_status ensure_desc(hmg_matrix* h, int elem)
     if (h->desc_near_mode == h->near_mode && h->desc_near_prec == h->near_prec &&
         h->desc_far_prec == h->far_prec && h->desc_elem == elem)
         return HMG_OK;
+    h->desc_near_mode = -1;  // a rebuild that fails half way leaves none
     const void* xs = elem == 8 ? (const void*)h->xs64 : (const void*)h->xs32;
     int near_esz = h->near_prec == HMG_PREC_FP64 ? 8 : 4;
     int far_esz = h->far_prec == HMG_PREC_FP64 ? 8 : 4;
