@@ -15,7 +15,7 @@ over 4,096 rows is reported beside every number (err_vs_fp64).
          in from the caller's pageable host memory and y copied out to it, every
          step, inside the timing.
   multi_rhs  products of 32 vectors a pass on the same H-matrix (hmg_matvec_multi,
-         CUDA cores), vectors per second.
+         straight from the storage), vectors per second.
   batched_tensor_cores  64 vectors a pass on the tensor cores with three-part BF16
          operands at N=2^18 (error <= 1e-6), beside the plain FP64 form at that size
          (the FP64 form of N=2^20 does not fit one B200).
@@ -683,7 +683,7 @@ def run_precision(a, rank, world):
             errs.append(float(torch.linalg.norm(Y[j][rows.long()] - yd) / torch.linalg.norm(yd)))
         info = H.info()
         if prec == hmg.PREC_FP32:
-            # tensor cores: BF16 factors with the near field in FP32 on the CUDA cores (the
+            # tensor cores: BF16 factors with the near field at FP32 accuracy (the
             # configuration as specified), then with the near field in BF16 as well
             tc = {}
             for near in (hmg.PREC_FP32, hmg.PREC_BF16):

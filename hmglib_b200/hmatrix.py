@@ -172,7 +172,7 @@ class HMatrix:
     def build_bf16_factors(self, near: int = L.PREC_BF16):
         """BF16 tcgen05 operands of the FP32 factors for tensor-core multi-vector products
         (hmg_build_tensor_core_operands); the near field on the tensor cores too
-        (near=PREC_BF16), in FP32 on the CUDA cores (near=PREC_FP32), or every operand
+        (near=PREC_BF16), at FP32 accuracy from the storage (near=PREC_FP32), or every operand
         as a BF16 hi + lo pair (near=PREC_BF16X3, ~5e-6) or as three BF16 parts
         (near=PREC_BF16X6, 24 bits)."""
         self._call("hmg_build_tensor_core_operands", int(near))
@@ -190,7 +190,7 @@ class HMatrix:
 
     def set_tensor_core_min_vectors(self, nrhs: int):
         """With on-chip tensor-core operands, multi-vector products of fewer than nrhs
-        vectors (default 17) run on the CUDA cores (hmg_set_tensor_core_min_vectors)."""
+        vectors (default 17) run from the storage (hmg_set_tensor_core_min_vectors)."""
         self._call("hmg_set_tensor_core_min_vectors", int(nrhs))
 
     def set_product_precision(self, precision: int):

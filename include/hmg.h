@@ -164,7 +164,7 @@ hmg_status hmg_full_matvec_rows(hmg_matrix* h, const double* x, const int* rows,
  * field (hmg_precompute_dense with HMG_PREC_FP32) too.  Afterwards hmg_matvec_multi
  * with 2..64 vectors computes t_b = V_b^T X_b and U t_b on the tensor cores with BF16
  * operands (X and t_b rounded to BF16) and FP32 accumulation; the near field runs
- * there as well (HMG_PREC_BF16) or on the CUDA cores in FP32 (HMG_PREC_FP32).  Results
+ * there as well (HMG_PREC_BF16) or at FP32 accuracy from the storage (HMG_PREC_FP32).  Results
  * agree with the FP32 products to ~1e-3 (BF16 rounding).  HMG_PREC_BF16X3 keeps every
  * operand, the near field included, as a BF16 pair (hi and the rounding of what hi
  * misses) and multiplies hi*hi + hi*lo + lo*hi: ~7e-6, with twice the operand bytes
@@ -182,7 +182,7 @@ hmg_status hmg_full_matvec_rows(hmg_matrix* h, const double* x, const int* rows,
  * MMAs).  Products agree with FP64 to ~4e-7 like HMG_PREC_BF16X6, and the only memory
  * added is the X and t_b operand buffer (3 x 2 bytes x 64 vectors per column and per
  * term): this is the form that fits at N = 2^20.  Its products of fewer than 17
- * vectors a pass run on the CUDA cores (hmg_set_tensor_core_min_vectors).  The plan
+ * vectors a pass run straight from the storage (hmg_set_tensor_core_min_vectors).  The plan
  * is built on the host once, on several threads.
  * hmg_build_bf16_factors(h) is hmg_build_tensor_core_operands(h, HMG_PREC_BF16). */
 hmg_status hmg_build_tensor_core_operands(hmg_matrix* h, int near_precision);
@@ -316,10 +316,10 @@ hmg_status hmg_autotune(hmg_matrix* h, int reps, int* piece_bytes, int* ctas_per
 hmg_status hmg_set_graphs(hmg_matrix* h, int on);
 
 /* Multi-vector products on a handle with operands converted on chip
- * (hmg_build_tensor_core_operands with HMG_PREC_BF16X6_ONCHIP) run on the tensor
- * cores from nrhs vectors a pass (default 17); smaller batches run on the CUDA
- * cores, which are faster there: a tensor-core pass costs about the same for 2 to
- * 32 vectors.  nrhs >= 2; 2 sends every multi-vector product to the tensor cores.
+ * (hmg_build_tensor_core_operands with HMG_PREC_BF16X6_ONCHIP) use those operands
+ * from nrhs vectors a pass (default 17); smaller batches run straight from the
+ * storage, which is faster there: a pass over the operands costs about the same for
+ * 2 to 32 vectors.  nrhs >= 2; 2 sends every multi-vector product to the operands.
  * No reference counterpart (the reference multiplies one vector per call). */
 hmg_status hmg_set_tensor_core_min_vectors(hmg_matrix* h, int nrhs);
 
