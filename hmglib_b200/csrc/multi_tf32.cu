@@ -894,6 +894,10 @@ hmg_status matvec_multi_tf32(hmg_matrix* h, int nrhs, const double* X, int ldx, 
 // tensor-core path with its near field in FP32).  xm: n2 x 32 values and a flag.
 hmg_status near_multi32(hmg_matrix* h, const double* X, int ldx, int nrhs, float* xm, double* Y, int ldy)
 {
+    // a product in another near-field mode or arithmetic may have left other descriptors, and
+    // one that ran out of memory none
+    hmg_status st = ensure_desc(h, 4);
+    if (st) return st;
     int* wide = reinterpret_cast<int*>(xm + (size_t)h->n[1] * 32);
     HMG_CUDA_TRY(cudaMemsetAsync(wide, 0, sizeof(int), h->stream));
     k_gather_tf32<<<ceil_div((long long)h->n[1] * 32, 256), 256, 0, h->stream>>>(X, ldx, nrhs, h->perm[1], h->n[1], 32,
