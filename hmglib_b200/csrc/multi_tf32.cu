@@ -115,7 +115,9 @@ template <int NT> struct FragB {
 
 // The split of an infinity or a NaN is not one (inf - inf), nor is that of a value which
 // rounds to infinity.  The kernels that write vectors set a flag where one is at or above
-// TF32_MAX, and the ones that read them then multiply with FP32 multiply-adds (step_fma).
+// TF32_MAX (wide[0]: X, wide[1]: t), and the kernels launched after them, which read these
+// vectors, then multiply with FP32 multiply-adds (step_fma).  No kernel reads a flag that it
+// sets: its warps would disagree.
 __device__ __forceinline__ bool splits(float v) { return fabsf(v) < __uint_as_float(TF32_MAX_BITS); }
 
 // acc[j] += A B_j for one K step: FP32 values (three MMAs) or values that are TF32 (two)
@@ -259,7 +261,7 @@ k_vtx_tf32(const VtTask* __restrict__ tasks, int nlarge, int nsmall, const float
         }
     };
     const int ntask = nlarge + nsmall;
-    const bool plain = *static_cast<volatile int*>(wide) != 0;  // (set here too: see splits)
+    const bool plain = wide[0] != 0;
     const double untruncate = plain ? 1.0 : UNTRUNCATE;
     bool fits = true;
 
@@ -476,7 +478,7 @@ k_vtx_tf32(const VtTask* __restrict__ tasks, int nlarge, int nsmall, const float
     if (plain) run(std::true_type{});
     else run(std::false_type{});
     cp_wait<0>();
-    if (!fits) *wide = 1;
+    if (!fits) wide[1] = 1;
 }
 
 struct VtItem {
@@ -599,7 +601,7 @@ k_tile_tf32(const PairDesc* __restrict__ desc, const int* tile_pair_start, const
     char* ring = tt_smem + (size_t)warp * NS * S::STAGE;
     const uint32_t ring_s = static_cast<uint32_t>(__cvta_generic_to_shared(ring));
     const int pend = g < G ? tile_pair_start[t + 1] : 0;
-    const bool plain = *wide != 0;
+    const bool plain = (wide[0] | wide[1]) != 0;
     const double untruncate = plain ? 1.0 : UNTRUNCATE;
 
     // producer: pair; within it the tier (0 FP32, 1 FP16, 2 FP8), the lane's next slice and
@@ -863,13 +865,13 @@ hmg_status matvec_multi_tf32(hmg_matrix* h, int nrhs, const double* X, int ldx, 
     if ((st = ensure_desc(h, 4)) || (st = ensure_vt(h))) return st;
     float* xm = nullptr;
     float* tm = nullptr;
-    // the flag of values the split does not take sits behind xm
-    if ((st = dalloc(&xm, (size_t)h->n[1] * R + 1, s)) || (st = dalloc(&tm, (size_t)(h->rank_total + 1) * R, s))) {
+    // the flags of values the split does not take sit behind xm
+    if ((st = dalloc(&xm, (size_t)h->n[1] * R + 2, s)) || (st = dalloc(&tm, (size_t)(h->rank_total + 1) * R, s))) {
         dfree(xm, s);
         return st;
     }
     int* wide = reinterpret_cast<int*>(xm + (size_t)h->n[1] * R);
-    cudaError_t e = cudaMemsetAsync(wide, 0, sizeof(int), s);
+    cudaError_t e = cudaMemsetAsync(wide, 0, 2 * sizeof(int), s);
     if (e == cudaSuccess) {
         k_gather_tf32<<<ceil_div((long long)h->n[1] * R, 256), 256, 0, s>>>(X, ldx, nrhs, h->perm[1], h->n[1], R, xm, wide);
         e = cudaGetLastError();
@@ -891,7 +893,7 @@ hmg_status matvec_multi_tf32(hmg_matrix* h, int nrhs, const double* X, int ldx, 
 }
 
 // Y = the near-field part of H X for up to 32 vectors, FP32 stored near field (the BF16
-// tensor-core path with its near field in FP32).  xm: n2 x 32 values and a flag.
+// tensor-core path with its near field in FP32).  xm: n2 x 32 values and two flags.
 hmg_status near_multi32(hmg_matrix* h, const double* X, int ldx, int nrhs, float* xm, double* Y, int ldy)
 {
     // a product in another near-field mode or arithmetic may have left other descriptors, and
@@ -899,7 +901,7 @@ hmg_status near_multi32(hmg_matrix* h, const double* X, int ldx, int nrhs, float
     hmg_status st = ensure_desc(h, 4);
     if (st) return st;
     int* wide = reinterpret_cast<int*>(xm + (size_t)h->n[1] * 32);
-    HMG_CUDA_TRY(cudaMemsetAsync(wide, 0, sizeof(int), h->stream));
+    HMG_CUDA_TRY(cudaMemsetAsync(wide, 0, 2 * sizeof(int), h->stream));
     k_gather_tf32<<<ceil_div((long long)h->n[1] * 32, 256), 256, 0, h->stream>>>(X, ldx, nrhs, h->perm[1], h->n[1], 32,
                                                                                 xm, wide);
     HMG_LAUNCH_CHECK();

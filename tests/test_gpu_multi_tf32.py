@@ -100,3 +100,26 @@ def test_zero_vectors_and_a_later_finite_product(hmg, cuda):
     torch.cuda.synchronize()
     assert torch.equal(A, B)
     H.close()
+
+
+@pytest.mark.parametrize("storage", ["fp32", "mixed"])
+def test_sums_that_overflow_on_the_way(hmg, cuda, storage):
+    """Vectors near the FP32 limit whose V^T x overflows in some blocks while others are still
+    being multiplied: every product of the same vectors is the same, bit for bit, and its other
+    vectors keep their values."""
+    torch = cuda
+    H, n = _build(hmg, "uniform", 9000, 2, 64, hmg.PREC_MIXED if storage == "mixed" else hmg.PREC_FP32)
+    X = torch.from_numpy(np.random.default_rng(3).uniform(-1, 1, (9, n))).cuda()
+    Y0 = torch.empty_like(X)
+    H.matvec_multi(X, Y0)
+    X[4] = 2e36  # finite, and so is its TF32 rounding; sums of 200 of them are not
+    Y, Z = torch.empty_like(X), torch.empty_like(X)
+    H.matvec_multi(X, Y)
+    for _ in range(20):
+        H.matvec_multi(X, Z)
+        torch.cuda.synchronize()
+        assert torch.equal(Y.nan_to_num(nan=7.0), Z.nan_to_num(nan=7.0)) and torch.equal(Y.isnan(), Z.isnan())
+    assert not bool(torch.isfinite(Y[4]).all())
+    for j in (0, 8):
+        assert rel_err(Y[j].cpu().numpy(), Y0[j].cpu().numpy()) < 1e-6
+    H.close()
