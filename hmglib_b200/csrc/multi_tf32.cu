@@ -265,12 +265,13 @@ k_vtx_tf32(const VtTask* __restrict__ tasks, int nlarge, int nsmall, const float
     const double untruncate = plain ? 1.0 : UNTRUNCATE;
     bool fits = true;
 
-    // producer: the lane's rows of the task (offsets from the block's V, a bit per row that
-    // exists), its X rows, and the step
+    // producer: the lane's rows of the task (offsets from the block's V, which may pass 4 GiB,
+    // a bit per row that exists), its X rows, and the step
     int pt = first_task(), left = 0, cleft = 0, xleft = 0, nload = 0;
     const char* vp = nullptr;   // the lane's chunk of the next step, row 0
     const float* xp = nullptr;  // X row of the next step's first column
-    uint32_t off[VT_LD], rows = 0;
+    size_t off[VT_LD];
+    uint32_t rows = 0;
     uint32_t xdst[NT];
     int xsrc[NT], xcol[NT];
 #pragma unroll
@@ -308,7 +309,7 @@ k_vtx_tf32(const VtTask* __restrict__ tasks, int nlarge, int nsmall, const float
                 r = p.n32 + (p.n16 >> 1) + (mt - nm32 - nm16) * 4 + (lg >> 1);
                 end = p.n32 + (p.n16 >> 1) + (p.n8 >> 2);
             }
-            off[i] = (uint32_t)r * (uint32_t)(p.chunks * 16);
+            off[i] = (size_t)r * p.chunks * 16;
             if (r < end) rows |= 1u << i;
         }
     };
