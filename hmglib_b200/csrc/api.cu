@@ -70,7 +70,7 @@ hmg_status hmg_create(hmg_matrix** out, int n1, int n2, int dim, int bits, void*
         delete h;
         return HMG_ERR_CUDA;
     }
-    pool_retain(h->device);
+    h->pool_generation = pool_retain(h->device);
     hmg_status st = dalloc(&h->dev_err, 4, h->stream);  // [0] error flag, [1],[2] work counters
     if (!st && cudaMemsetAsync(h->dev_err, 0, 4 * sizeof(int), h->stream) != cudaSuccess) st = HMG_ERR_CUDA;
     for (int i = 0; i < 2 && !st; i++) {
@@ -86,7 +86,7 @@ hmg_status hmg_create(hmg_matrix** out, int n1, int n2, int dim, int bits, void*
     }
     if (st) {
         free_matrix_buffers(h);
-        pool_release(h->device);
+        pool_release(h->device, h->pool_generation);
         delete h;
         return st;
     }
@@ -477,7 +477,7 @@ hmg_status hmg_destroy(hmg_matrix* h)
         if (h->k1_ev[i]) cudaEventDestroy(h->k1_ev[i]);
     free_matrix_buffers(h);
     cudaStreamSynchronize(h->stream);
-    pool_release(h->device);
+    pool_release(h->device, h->pool_generation);
     delete h;
     return HMG_OK;
 }

@@ -7,6 +7,8 @@
 // Passes whose digit is identical for every key are skipped (decided from one
 // up-front histogram of all eight digits), which is exact and removes the top
 // pass of 3D codes (60 significant bits).
+#include <cuda.h>
+
 #include <cstdarg>
 #include <mutex>
 
@@ -213,26 +215,69 @@ hmg_status radix_sort_pairs(uint64_t* keys, uint32_t* vals, int n, int key_bits,
 // the library's device pools
 // ---------------------------------------------------------------------------
 static constexpr int POOL_DEVICES = 64;
+struct DevicePool {
+    cudaMemPool_t pool = nullptr;
+    unsigned long long context = 0;  // the primary context it was created in
+    bool tried = false;
+    int users = 0;                   // live handles of that context
+    unsigned generation = 0;         // contexts seen
+};
 static std::mutex g_pool_mutex;
-static cudaMemPool_t g_pool[POOL_DEVICES];
-static bool g_pool_tried[POOL_DEVICES];
-static int g_pool_users[POOL_DEVICES];  // live handles
+static DevicePool g_pool[POOL_DEVICES];
 
-static cudaMemPool_t pool_of(int device)  // g_pool_mutex held
+// The unique id of the current device's primary context, which cudaDeviceReset ends: the
+// next one has another id.  0 if the driver cannot say.
+static unsigned long long context_id(int device)
+{
+    typedef CUresult (*CtxGetCurrent)(CUcontext*);
+    typedef CUresult (*CtxGetId)(CUcontext, unsigned long long*);
+    struct Driver {
+        CtxGetCurrent current = nullptr;
+        CtxGetId id = nullptr;
+        Driver()
+        {
+            void *c = nullptr, *i = nullptr;
+            cudaDriverEntryPointQueryResult q;
+            if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &c, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+                cudaGetDriverEntryPointByVersion("cuCtxGetId", &i, 12000, cudaEnableDefault, &q) == cudaSuccess) {
+                current = reinterpret_cast<CtxGetCurrent>(c);
+                id = reinterpret_cast<CtxGetId>(i);
+            } else {
+                cudaGetLastError();
+            }
+        }
+    };
+    static const Driver driver;
+    if (!driver.current || !driver.id) return 0;
+    for (int attempt = 0; attempt < 2; attempt++) {
+        CUcontext c = nullptr;
+        unsigned long long id = 0;
+        if (driver.current(&c) == CUDA_SUCCESS && c && driver.id(c, &id) == CUDA_SUCCESS) return id;
+        // none yet in this thread, or one that a reset ended: the runtime makes the next
+        if (cudaSetDevice(device) != cudaSuccess) cudaGetLastError();
+    }
+    return 0;
+}
+
+// The entry of the current device; g_pool_mutex held.  A pool of a context that
+// cudaDeviceReset has ended is gone: it is dropped, not destroyed, and made anew.
+static DevicePool* pool_of(int device)
 {
     if (device < 0 || device >= POOL_DEVICES) return nullptr;
-    if (!g_pool_tried[device]) {
-        g_pool_tried[device] = true;
+    DevicePool& p = g_pool[device];
+    const unsigned long long context = context_id(device);
+    if (!p.tried || p.context != context) {
+        p = DevicePool{nullptr, context, true, 0, p.generation + 1};
         cudaMemPoolProps props{};
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = device;
-        if (cudaMemPoolCreate(&g_pool[device], &props) != cudaSuccess) {
+        if (cudaMemPoolCreate(&p.pool, &props) != cudaSuccess) {
             cudaGetLastError();
-            g_pool[device] = nullptr;
+            p.pool = nullptr;
         }
     }
-    return g_pool[device];
+    return &p;
 }
 
 cudaMemPool_t device_pool()
@@ -243,7 +288,8 @@ cudaMemPool_t device_pool()
         return nullptr;
     }
     std::lock_guard<std::mutex> lock(g_pool_mutex);
-    return pool_of(device);
+    const DevicePool* p = pool_of(device);
+    return p ? p->pool : nullptr;
 }
 
 // bytes the pool keeps mapped at a synchronisation
@@ -252,20 +298,30 @@ static void pool_keep(cudaMemPool_t pool, unsigned long long bytes)
     if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &bytes) != cudaSuccess) cudaGetLastError();
 }
 
-void pool_retain(int device)
+unsigned pool_retain(int device)
 {
     std::lock_guard<std::mutex> lock(g_pool_mutex);
-    const cudaMemPool_t pool = pool_of(device);
-    if (pool && g_pool_users[device]++ == 0) pool_keep(pool, POOL_KEEP);
+    DevicePool* p = pool_of(device);
+    if (!p || !p->pool) return 0;
+    if (p->users++ == 0) pool_keep(p->pool, POOL_KEEP);
+    return p->generation;
 }
 
-void pool_release(int device)
+void pool_release(int device, unsigned generation)
 {
-    std::lock_guard<std::mutex> lock(g_pool_mutex);
-    const cudaMemPool_t pool = pool_of(device);
-    if (!pool || --g_pool_users[device] > 0) return;
-    pool_keep(pool, 0);
-    if (cudaMemPoolTrimTo(pool, 0) != cudaSuccess) cudaGetLastError();
+    if (!generation) return;
+    int current = device;
+    if (cudaGetDevice(&current) != cudaSuccess) cudaGetLastError();
+    if (current != device && cudaSetDevice(device) != cudaSuccess) cudaGetLastError();
+    {
+        std::lock_guard<std::mutex> lock(g_pool_mutex);
+        DevicePool* p = pool_of(device);
+        if (p && p->generation == generation && --p->users == 0) {
+            pool_keep(p->pool, 0);
+            if (cudaMemPoolTrimTo(p->pool, 0) != cudaSuccess) cudaGetLastError();
+        }
+    }
+    if (current != device && cudaSetDevice(current) != cudaSuccess) cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------

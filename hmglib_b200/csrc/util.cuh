@@ -13,11 +13,12 @@ namespace hmg {
 // default pool, which other code may share and whose settings stay untouched, unmaps
 // everything free at every synchronisation: about 0.2 ms to map and 0.2 ms to unmap a
 // small block, 6.3 ms a GB each way (measured on a B200), in a setup that synchronises
-// some twenty times.  Thread-safe.
+// some twenty times.  Thread-safe.  A cudaDeviceReset ends the pool with its context: the
+// next use makes another, and handles of the old context (their generation) no longer count.
 static constexpr unsigned long long POOL_KEEP = 1ull << 30;
 cudaMemPool_t device_pool();
-void pool_retain(int device);
-void pool_release(int device);
+unsigned pool_retain(int device);  // the current device; returns the pool's generation (0: no pool)
+void pool_release(int device, unsigned generation);
 
 // Stream-ordered device allocation helpers.
 template <typename T>

@@ -98,6 +98,10 @@ int hmg_version(void);
  * dimensions; `bits` is the Morton resolution per dimension (0 picks 32 for 2D,
  * 20 for 3D, the only pairs the reference supports, morton.cu:21-67).
  * `stream` is a cudaStream_t (NULL = default stream).
+ * Temporary device memory comes from a stream-ordered pool of the library's own, one a
+ * device.  While a handle lives it keeps up to 1 GB of freed memory mapped; the last
+ * hmg_destroy gives it back.  cudaDeviceReset ends the pool with every handle of the
+ * context; handles created afterwards use a new one.
  * Replaces init_h_matrix_data (hmglib.cu:68-123). */
 hmg_status hmg_create(hmg_matrix** out, int n1, int n2, int dim, int bits, void* stream);
 
