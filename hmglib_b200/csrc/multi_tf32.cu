@@ -544,11 +544,15 @@ static hmg_status ensure_vt(hmg_matrix* h)
             dfree(t, s);
             return st;
         }
-        if (cudaMemcpyAsync(d, large.data(), sizeof(VtItem) * n, cudaMemcpyHostToDevice, s) == cudaSuccess)
+        cudaError_t e = cudaMemcpyAsync(d, large.data(), sizeof(VtItem) * n, cudaMemcpyHostToDevice, s);
+        if (e == cudaSuccess) {
             k_build_vt<<<ceil_div(n, 256), 256, 0, s>>>(d, n, h->blk_c0, h->blk_m2, h->rank, h->tier32, h->tier16,
                                                         h->rank_off, h->ptrV, mixed ? 1 : 0, t);
+            e = cudaGetLastError();
+        }
         dfree(d, s);
-        const cudaError_t e = cudaStreamSynchronize(s);  // the host vector goes out of scope
+        const cudaError_t done = cudaStreamSynchronize(s);  // the host vector goes out of scope
+        if (e == cudaSuccess) e = done;
         if (e != cudaSuccess) {
             dfree(t, s);
             set_error("building the V^T X tasks failed: %s", cudaGetErrorString(e));

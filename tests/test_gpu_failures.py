@@ -93,3 +93,30 @@ def test_near_mode_changed_between_products(hmg, cuda):
     assert rel_err(B[0].cpu().numpy(), fp64_rows(torch, H, X[0].contiguous(), np.arange(n))) < 5e-3
     assert torch.equal(A, B)
     H.close()
+
+
+def test_tasks_after_a_failed_copy(hmg, cuda, faulty):
+    """The first multi-vector product cannot copy its task list to the device: it fails, and the
+    next one builds the list instead of using the uninitialised one."""
+    torch = cuda
+    n = 6000
+    p = make_points("uniform", n, 2, 5)
+    out = []
+    for fail in (False, True):
+        H = engine(hmg, p, p, 1.5, 64, rule=1)
+        H.set_kernel(3, 0.05, 0.0)
+        H.precompute_aca(64, 1e-8, hmg.PREC_FP32)
+        H.precompute_dense(hmg.PREC_FP32)
+        X = torch.from_numpy(np.random.default_rng(2).uniform(-1, 1, (3, n))).cuda()
+        Y = torch.full_like(X, float("nan"))
+        H.matvec(X[0], Y[0])  # the descriptors are there
+        if fail:
+            faulty(COPY, 0)
+            with pytest.raises(hmg.HmgError):
+                H.matvec_multi(X, Y)
+            faulty(COPY, -1)
+        H.matvec_multi(X, Y)
+        torch.cuda.synchronize()
+        out.append(Y)
+        H.close()
+    assert torch.equal(*out)
