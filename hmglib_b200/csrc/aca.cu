@@ -923,6 +923,58 @@ void free_far(hmg_matrix* h)
     h->h_rank.clear();
 }
 
+// Scratch of the batches, grown to the largest batch and reused across batches; however
+// run_aca returns, its kernels have ended and the scratch is given back.  The factors' part
+// is up to 4 GB, which the stream-ordered pool maps and unmaps at 6.3 ms a GB each way; a
+// cudaMalloc and its cudaFree take 0.7 ms and 0.8 more a GB (measured), so from 64 MB on it
+// comes from there.  (cudaFree waits for the device; products on another stream beside
+// builds of 131,072 points: p50 1.60 ms with pool scratch, 1.78 now, p99 115 and 36 ms.)
+struct AcaScratch {
+    static constexpr size_t POOLED = (64u << 20) / sizeof(double);
+    hmg_matrix* h;
+    double* uv = nullptr;  // the batch's u terms, then its v terms
+    size_t cap_uv = 0;
+    int *idx = nullptr, *rank = nullptr, *r32 = nullptr, *r16 = nullptr, *list = nullptr;
+    long long *uo = nullptr, *vo = nullptr, *so = nullptr;
+    double *s2 = nullptr, *tn = nullptr;
+    float *su = nullptr, *sv = nullptr;
+
+    explicit AcaScratch(hmg_matrix* m) : h(m) {}
+    AcaScratch(const AcaScratch&) = delete;
+    AcaScratch& operator=(const AcaScratch&) = delete;
+    ~AcaScratch() { release(); }
+    void release()
+    {
+        const cudaStream_t s = h->stream;
+        for (cudaStream_t aux : h->k1_aux)
+            if (aux) cudaStreamSynchronize(aux);
+        cudaStreamSynchronize(s);
+        drop();
+        dfree(idx, s); dfree(rank, s); dfree(r32, s); dfree(r16, s); dfree(list, s);
+        dfree(uo, s); dfree(vo, s); dfree(so, s);
+        dfree(s2, s); dfree(tn, s); dfree(su, s); dfree(sv, s);
+    }
+    void drop()
+    {
+        if (cap_uv <= POOLED) dfree(uv, h->stream);
+        else if (uv) cudaFree(uv);
+        uv = nullptr;
+        cap_uv = 0;
+    }
+    hmg_status grow(size_t n)
+    {
+        drop();
+        cap_uv = n > 0 ? n : 1;
+        if (cap_uv <= POOLED) return dalloc(&uv, cap_uv, h->stream);
+        const cudaError_t e = cudaMalloc((void**)&uv, cap_uv * sizeof(double));
+        if (e == cudaSuccess) return HMG_OK;
+        cudaGetLastError();
+        uv = nullptr;
+        set_error("allocating %zu bytes of ACA scratch failed: %s", cap_uv * sizeof(double), cudaGetErrorString(e));
+        return e == cudaErrorMemoryAllocation ? HMG_ERR_NOMEM : HMG_ERR_CUDA;
+    }
+};
+
 hmg_status run_aca(hmg_matrix* h, int k, double eps, int precision)
 {
     cudaStream_t s = h->stream;
@@ -966,41 +1018,12 @@ hmg_status run_aca(hmg_matrix* h, int k, double eps, int precision)
     P.n1 = h->n[0];
     P.n2 = h->n[1];
 
-    // Scratch of the batches, grown to the largest batch and reused across batches.  The
-    // factors' part is up to 4 GB, which the stream-ordered pool maps and unmaps at 6.3 ms a
-    // GB each way; a cudaMalloc and its cudaFree take 0.7 ms and 0.8 more a GB (measured), so
-    // from 64 MB on it comes from there.
-    static constexpr size_t POOL_SCRATCH = (64u << 20) / sizeof(double);
-    int* d_idx = nullptr;
-    long long *d_uo = nullptr, *d_vo = nullptr, *d_so = nullptr;
-    double *dU = nullptr, *d_s2 = nullptr, *d_tn = nullptr;  // dU: the batch's u terms, then its v terms
-    int *d_rank = nullptr, *d_r32 = nullptr, *d_r16 = nullptr, *d_list = nullptr;
-    float *d_su = nullptr, *d_sv = nullptr;
-    size_t cap_ne = 0, cap_uv = 0, cap_sc = 0;
-    auto drop = [&]() {
-        if (cap_uv <= POOL_SCRATCH) dfree(dU, s);
-        else if (dU) cudaFree(dU);
-        dU = nullptr;
-        cap_uv = 0;
-    };
-    auto grow = [&](size_t n) {
-        drop();
-        cap_uv = n > 0 ? n : 1;
-        if (cap_uv <= POOL_SCRATCH) return dalloc(&dU, cap_uv, s);
-        const cudaError_t e = cudaMalloc((void**)&dU, cap_uv * sizeof(double));
-        if (e == cudaSuccess) return HMG_OK;
-        cudaGetLastError();
-        dU = nullptr;
-        set_error("allocating %zu bytes of ACA scratch failed: %s", cap_uv * sizeof(double), cudaGetErrorString(e));
-        return e == cudaErrorMemoryAllocation ? HMG_ERR_NOMEM : HMG_ERR_CUDA;
-    };
-    auto free_batch = [&]() {
-        drop();
-        dfree(d_idx, s); dfree(d_uo, s); dfree(d_vo, s);
-        dfree(d_rank, s); dfree(d_s2, s); dfree(d_so, s); dfree(d_r32, s); dfree(d_r16, s);
-        dfree(d_su, s); dfree(d_sv, s); dfree(d_tn, s); dfree(d_list, s);
-        cap_ne = cap_sc = 0;
-    };
+    AcaScratch W(h);
+    int *&d_idx = W.idx, *&d_rank = W.rank, *&d_r32 = W.r32, *&d_r16 = W.r16, *&d_list = W.list;
+    long long *&d_uo = W.uo, *&d_vo = W.vo, *&d_so = W.so;
+    double *&dU = W.uv, *&d_s2 = W.s2, *&d_tn = W.tn;
+    float *&d_su = W.su, *&d_sv = W.sv;
+    size_t cap_ne = 0, cap_sc = 0;
     int bstart = h->ndense;
     while (bstart < nb) {
         std::vector<int> idx;
@@ -1035,24 +1058,17 @@ hmg_status run_aca(hmg_matrix* h, int k, double eps, int precision)
             if ((st = dalloc(&d_idx, cap_ne, s)) || (st = dalloc(&d_uo, cap_ne, s)) || (st = dalloc(&d_vo, cap_ne, s)) ||
                 (st = dalloc(&d_rank, cap_ne, s)) || (st = dalloc(&d_s2, cap_ne, s)) || (st = dalloc(&d_list, cap_ne, s)) ||
                 (mixed && ((st = dalloc(&d_so, cap_ne, s)) || (st = dalloc(&d_r32, cap_ne, s)) ||
-                           (st = dalloc(&d_r16, cap_ne, s))))) {
-                free_batch();
+                           (st = dalloc(&d_r16, cap_ne, s)))))
                 return st;
-            }
         }
-        if ((size_t)(us + vs) > cap_uv && (st = grow((size_t)(us + vs)))) {
-            free_batch();
-            return st;
-        }
+        if ((size_t)(us + vs) > W.cap_uv && (st = W.grow((size_t)(us + vs)))) return st;
         if (mixed && (size_t)nscale > cap_sc) {
             dfree(d_su, s);
             dfree(d_sv, s);
             dfree(d_tn, s);
             cap_sc = (size_t)nscale;
-            if ((st = dalloc(&d_su, cap_sc, s)) || (st = dalloc(&d_sv, cap_sc, s)) || (st = dalloc(&d_tn, 3 * cap_sc, s))) {
-                free_batch();
+            if ((st = dalloc(&d_su, cap_sc, s)) || (st = dalloc(&d_sv, cap_sc, s)) || (st = dalloc(&d_tn, 3 * cap_sc, s)))
                 return st;
-            }
         }
         HMG_CUDA_TRY(cudaMemcpyAsync(d_idx, idx.data(), sizeof(int) * ne, cudaMemcpyHostToDevice, s));
         HMG_CUDA_TRY(cudaMemcpyAsync(d_uo, uo.data(), sizeof(long long) * ne, cudaMemcpyHostToDevice, s));
@@ -1063,7 +1079,6 @@ hmg_status run_aca(hmg_matrix* h, int k, double eps, int precision)
         const size_t mask = eps > 0.0 ? ((size_t)((maxm1 + 31) / 32) * 4 + 7) & ~(size_t)7 : 0;
         if (mask > 200 * 1024) {
             set_error("block with %d rows exceeds the adaptive ACA's row-mask capacity", maxm1);
-            free_batch();
             return HMG_ERR_UNSUPPORTED;
         }
         // the blocks by class, in each the ones with most work first
@@ -1089,10 +1104,7 @@ hmg_status run_aca(hmg_matrix* h, int k, double eps, int precision)
         const bool fork = us + vs > (16ll << 20);
         cudaStream_t on[ACA_NCLASS] = {s, s, s, s};
         if (fork) {
-            if ((st = ensure_side_streams(h))) {
-                free_batch();
-                return st;
-            }
+            if ((st = ensure_side_streams(h))) return st;
             HMG_CUDA_TRY(cudaEventRecord(h->k1_ev[0], s));
             for (int i = 0; i < 2; i++) HMG_CUDA_TRY(cudaStreamWaitEvent(h->k1_aux[i], h->k1_ev[0], 0));
             on[0] = on[2] = h->k1_aux[0];
@@ -1104,11 +1116,8 @@ hmg_status run_aca(hmg_matrix* h, int k, double eps, int precision)
         if ((st = launch_aca<512, 2, 1>(g, h->kspec, P, B, k, eps, d_list + first[3], count[3], big, kc(3), bits(3), s)) ||
             (st = launch_aca<512, 1, 2>(g, h->kspec, P, B, k, eps, d_list + first[2], count[2], ACA_CLASSES[2].panel, kc(2), bits(2), on[2])) ||
             (st = launch_aca<256, 1, 3>(g, h->kspec, P, B, k, eps, d_list + first[1], count[1], ACA_CLASSES[1].panel, kc(1), bits(1), on[1])) ||
-            (st = launch_small(g, h->kspec, P, B, k, eps, d_list + first[0], count[0], kc(0), bits(0), on[0]))) {
-            cudaDeviceSynchronize();
-            free_batch();
+            (st = launch_small(g, h->kspec, P, B, k, eps, d_list + first[0], count[0], kc(0), bits(0), on[0])))
             return st;
-        }
         for (int i = 0; i < 2 && fork; i++) {
             HMG_CUDA_TRY(cudaEventRecord(h->k1_ev[1 + i], h->k1_aux[i]));
             HMG_CUDA_TRY(cudaStreamWaitEvent(s, h->k1_ev[1 + i], 0));
@@ -1192,7 +1201,7 @@ hmg_status run_aca(hmg_matrix* h, int k, double eps, int precision)
         }
         HMG_CUDA_TRY(cudaStreamSynchronize(s));
     }
-    free_batch();
+    W.release();
 
     // ranks and their offsets
     std::vector<long long> roff(nb + 1, 0);

@@ -120,3 +120,53 @@ def test_tasks_after_a_failed_copy(hmg, cuda, faulty):
         out.append(Y)
         H.close()
     assert torch.equal(*out)
+
+
+@pytest.mark.parametrize("which", [MALLOC, POOL, COPY], ids=["malloc", "pool", "copy"])
+def test_construction_that_fails_gives_its_memory_back(hmg, cuda, faulty, which):
+    """hmg_precompute_aca with each of its allocations or copies failing in turn: it reports the
+    error, a retry on the same handle gives the factors of an undisturbed call, and with the
+    handle closed the device has all the memory that it had."""
+    torch = cuda
+    n = 20000
+    p = make_points("uniform", n, 3, 5)
+    x = torch.from_numpy(np.random.default_rng(2).uniform(-1, 1, n)).cuda()
+    y, ref = torch.empty_like(x), torch.empty_like(x)
+
+    def handle():
+        H = engine(hmg, p, p, 1.5, 64, rule=1)
+        H.set_kernel(4, 0.2, 0.0)
+        return H
+
+    def finish(H, out):
+        H.precompute_aca(96, 1e-6, hmg.PREC_MIXED)
+        H.precompute_dense(hmg.PREC_MIXED)
+        H.matvec(x, out)
+        torch.cuda.synchronize()
+        H.close()
+
+    finish(handle(), ref)
+    free, _ = torch.cuda.mem_get_info()
+    failed, after = 0, 0
+    while True:
+        H = handle()
+        faulty(which, after)
+        try:
+            H.precompute_aca(96, 1e-6, hmg.PREC_MIXED)
+            done = True
+        except hmg.HmgError as e:
+            done = False
+            failed += 1
+            assert which == COPY or e.status == 3, e  # HMG_ERR_NOMEM
+        faulty(which, -1)
+        if done:
+            H.close()
+            break
+        if after % 4 == 0:
+            finish(H, y)
+            assert torch.equal(y, ref)
+        else:
+            H.close()
+        assert torch.cuda.mem_get_info()[0] == free, after
+        after += 1
+    assert failed >= {MALLOC: 2, POOL: 10, COPY: 8}[which]
