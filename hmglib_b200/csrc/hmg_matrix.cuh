@@ -131,7 +131,7 @@ struct hmg_matrix {
     int k1_count[3] = {0, 0, 0};   // pieces per tier (FP32/FP64, FP16, FP8)
     int k1_piece_start[3][5] = {};  // per tier: first piece of each lane-group class, end
     int k1_task_start[3][5] = {};   // per tier: first warp task of each class, task count
-    void* vt_tasks = nullptr;      // multi-vector V^T X tasks (multi_tf32.cu), the split ones first
+    void* vt_tasks = nullptr;      // multi-vector V^T X tasks (multi_mma.cu), the split ones first
     int vt_large = 0, vt_small = 0;
     int* far_list = nullptr;       // admissible blocks with rank > 0 (streaming V^T x)
     int nfar_list = 0;
@@ -170,7 +170,7 @@ hmg_status ensure_side_streams(hmg_matrix* h);
 hmg_status matvec_device(hmg_matrix* h, const double* x, double* y, bool fp64_arith = false);
 hmg_status matvec_unbatched(hmg_matrix* h, const double* x, double* y);
 hmg_status matvec_multi(hmg_matrix* h, int nrhs, const double* X, int ldx, double* Y, int ldy);
-hmg_status matvec_multi_tf32(hmg_matrix* h, int nrhs, const double* X, int ldx, double* Y, int ldy);
+hmg_status matvec_multi_mma(hmg_matrix* h, int nrhs, const double* X, int ldx, double* Y, int ldy);
 hmg_status matvec_multi_tc(hmg_matrix* h, int nrhs, const double* X, int ldx, double* Y, int ldy);
 hmg_status build_bf16_factors(hmg_matrix* h, bool near_on_tensor_cores, int parts);
 hmg_status build_tcm(hmg_matrix* h);
@@ -179,6 +179,7 @@ void free_tcm(hmg_matrix* h);
 hmg_status autotune(hmg_matrix* h, int reps, int* best_piece, int* best_ctas, double* best_ms);
 void free_tc(hmg_matrix* h);
 void free_product_graph(hmg_matrix* h);
+static constexpr int MULTI_RANGE_WORDS = 33;  // behind the gathered vectors (multi_mma.cu)
 hmg_status near_multi32(hmg_matrix* h, const double* X, int ldx, int nrhs, float* xm, double* Y, int ldy);
 hmg_status direct_matvec(hmg_matrix* h, const double* x, const int* rows, int nrows,
                          double* y);

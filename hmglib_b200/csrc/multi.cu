@@ -5,7 +5,7 @@
 // a caller with several vectors pays the whole stored H-matrix once per vector.  Here
 // the factors and the near field are read once for all vectors: bytes per product are
 // those of one single-vector product plus 8 (N1 + N2) per vector, and each stored
-// value feeds nrhs multiply-adds.  FP32 and mixed storage: multi_tf32.cu.  FP64 storage,
+// value feeds nrhs multiply-adds.  FP32 and mixed storage: multi_mma.cu.  FP64 storage,
 // here: X (caller order, column-major) is gathered into Z order as R values per point
 // (R = nrhs rounded up to a power of two).
 //   K1m  t_b = V_b^T X_b for every admissible block: a warp per K1 piece; its lanes
@@ -216,7 +216,7 @@ hmg_status matvec_multi(hmg_matrix* h, int nrhs, const double* X, int ldx, doubl
         // one element type for the stored near field and the factors' FP32 / FP64 terms
         if (mixed ? h->ndense == 0 || h->near_prec == HMG_PREC_FP32
                   : h->near_prec == HMG_PREC_FP32 && (h->naca == 0 || h->far_prec == HMG_PREC_FP32))
-            return matvec_multi_tf32(h, nrhs, X, ldx, Y, ldy);
+            return matvec_multi_mma(h, nrhs, X, ldx, Y, ldy);
         if (!mixed && h->near_prec == HMG_PREC_FP64 && (h->naca == 0 || h->far_prec == HMG_PREC_FP64))
             return multi_fp64(h, nrhs, X, ldx, Y, ldy);
     }

@@ -1,29 +1,37 @@
-// multi_tf32.cu -- Y = H X for 2 to 32 vectors over FP32 or mixed storage, on the
+// multi_mma.cu -- Y = H X for 2 to 32 vectors over FP32 or mixed storage, on the
 // tensor cores with FP32 accuracy.
 //
 // The reference multiplies one vector per call (apply_h_matrix_mvp, hmglib.cu:271-286).
 // Here every stored value is read once for all vectors, straight into the fragments of
-// mma.sync m16n8k8 (TF32 operands, FP32 accumulator): the product is bound by the bytes
+// mma.sync m16n8k16 (BF16 operands, FP32 accumulator): the product is bound by the bytes
 // of the stored H-matrix, and a lane's own 16-byte loads already are its A fragments
 // (4 rows of a chunk column, or 4 columns of a V row), so no operand passes through a
 // shared tile or a descriptor.  The K order of an MMA is free as long as A and B agree:
 // each storage tier orders its terms so that the loads fit.
 //
-// FP32 accuracy from TF32 operands.  A value is split into its TF32 rounding and the
-// rest: rounding to nearest makes the rest signed, so what the third product's missing
-// lo*lo and the rest's last bit leave out has no bias.  FP32 x FP32 takes three MMAs
-// (lo*hi, hi*lo, hi*hi); FP16 and FP8 values are TF32 numbers and take two.  The
-// accumulator truncates, and a chain of truncations is biased, so a chain is one K step
-// of 8, smallest products first, from zero; the chains are added on the CUDA cores
-// (rounded to nearest).  Sums of 96 products then have a relative error of 1.1e-7 against
-// 64 bits (1.8e-7 for a chain of FP32 multiply-adds; 1.7e-7 with a truncated split).
+// FP32 accuracy from BF16 operands.  A value is cut into BF16 parts of 8 bits each, exactly:
+// three for FP32, two for FP16 and one for FP8.  All products of parts are formed but
+// tail x tail, at most 2^-32 of the whole.  The accumulator truncates, and a chain of
+// truncations is biased, so a chain is one step of 16 columns or terms: the heads' product
+// e from zero; its remainder (the heads once more, from -e) and the other products in two
+// chains, smallest first; these are added up, and added to the sum, on the CUDA cores
+// (rounded to nearest).  A head product has 16 bits, so what e and the remainder miss lies below 2^-24
+// of the step's largest product.  FP16 and FP8 terms, 1e-4 of a block and less, go without
+// the remainder.  Against 64 bits, sums of 96 products: 5.5e-8 relative, without a mean
+// shift, against 1.8e-7 for a chain of FP32 multiply-adds (values over a range of e^10, all
+// of one sign: 5.7e-8, 3.5e-8 of it low, against 1.5e-7); a product with a unit vector
+// returns the stored value.  Two TF32 parts and three products (6 MMAs for 16 columns, not
+// 9) lost the last bit of a quarter of the values and 4e-8 of every sum: unit vectors
+// were off by up to 1.6e-7, and CG on 8192 clustered points took 4785-4899 iterations instead
+// of 4571-4778.
 // Sums of a (tile, block) pair stay FP32 and pairs are added in FP64, as in the
 // single-vector product.  Deterministic.
 //
 // Measured at N = 2^17 (uniform 3D, Matern, mixed storage, 8.0 GB: 1.23 ms at the copy
 // peak) against the CUDA-core kernels (packed FP32 multiply-adds) this replaces: 8
-// vectors 2.83 ms (6.79), 16 3.93 (8.86), 32 7.0 (13.5).  Bound by instruction issue and
-// the latency of the MMA chains (tensor pipe 20-40 % busy), not by memory.
+// vectors 3.42 ms (7.18), 16 5.10 (9.45), 24 6.34 (14.1), 32 8.41 (14.1); with the two TF32
+// parts 2.77, 3.95, 5.16 and 6.94.  Bound by instruction issue and the latency of the MMA
+// chains, not by memory.
 #include <cuda_fp16.h>
 #include <cuda_fp8.h>
 
@@ -60,32 +68,31 @@ __device__ __forceinline__ void cp_vector16(uint32_t dst, const void* src, bool 
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// d = A B + c: A 16 x 8 (lane (g, t): rows g, g + 8 of column t, then of column t + 4),
-// B 8 x 8 (rows t, t + 4 of column g), d 16 x 8 (row g columns 2t, 2t + 1, then row g + 8)
-__device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2],
+// d = A B + c: A 16 x 16, B 16 x 8, d 16 x 8 (row g columns 2t, 2t + 1, then row g + 8).  A
+// register of A or B holds two K slots; lane (g, t) has A rows g, g + 8 and B column g.  The
+// kernels think of it as two K steps of 8: slot t or t + 4 (the register) of the first (its
+// low half) and of the second step (its high half).
+__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2],
                                          const float (&c)[4])
 {
-    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
         "{%10, %11, %12, %13};"
         : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "f"(c[0]), "f"(c[1]), "f"(c[2]), "f"(c[3]));
 }
 
-// The tensor core truncates a K step's sum: on average it is short by half a unit in the
-// last place, 4.0e-8 of itself (measured; 2^-24 / ln 4 = 4.3e-8 were the sum's mantissa
-// log-uniform).  Sums of steps are therefore scaled by this.  The shortfall has the sums'
-// sign, which neighbouring rows share: left in, it is a smooth error, which a CG solve's
-// residual cannot forget as it does rounding noise (4930 iterations instead of 4660 on 8192
-// clustered points, with smaller products' errors).
-static constexpr double UNTRUNCATE = 1.0 + 4.0e-8;
-
-// v as TF32, rounded to nearest (the tensor core drops the lower 13 bits), and the rest:
-// 11 bits of either sign, exact to one last bit of FP32.  |v| < TF32_MAX.
-static constexpr unsigned TF32_MAX_BITS = 0x7f7ff000u;
-__device__ __forceinline__ void tf32_split(uint32_t v, uint32_t& hi, uint32_t& lo)
+// The first PARTS runs of 8 bits of v0 and v1, as BF16 pairs (v0 in the low halves).  Cut,
+// not rounded: each rest is exact and three parts hold an FP32 value.
+template <int PARTS> __device__ __forceinline__ void split_pair(uint32_t v0, uint32_t v1, uint32_t (&p)[PARTS])
 {
-    hi = (v + 0x1000u) & 0xffffe000u;
-    lo = __float_as_uint(__uint_as_float(v) - __uint_as_float(hi));
+#pragma unroll
+    for (int i = 0; i < PARTS; i++) {
+        p[i] = __byte_perm(v0, v1, 0x7632);
+        if (i + 1 < PARTS) {
+            v0 = __float_as_uint(__uint_as_float(v0) - __uint_as_float(v0 & 0xffff0000u));
+            v1 = __float_as_uint(__uint_as_float(v1) - __uint_as_float(v1 & 0xffff0000u));
+        }
+    }
 }
 
 // acc += d, two lanes of FP32 at a time
@@ -98,58 +105,94 @@ __device__ __forceinline__ void add4(float (&acc)[4], const float (&d)[4])
         : "f"(d[0]), "f"(d[1]), "f"(d[2]), "f"(d[3]));
 }
 
-// The B fragments of one K step for NT groups of 8 vectors, split.
+// The B fragments of a step for NT groups of 8 vectors, split: rows (lo0, hi0) and (lo1, hi1)
+// are the K slots of its two registers.
 template <int NT> struct FragB {
-    uint32_t hi[NT][2], lo[NT][2];
-    __device__ __forceinline__ void get(const float* b0, const float* b1)
+    uint32_t p[3][NT][2];
+    __device__ __forceinline__ void get(const float* lo0, const float* lo1, const float* hi0, const float* hi1)
     {
 #pragma unroll
-        for (int j = 0; j < NT; j++) {
-            tf32_split(__float_as_uint(b0[8 * j]), hi[j][0], lo[j][0]);
-            tf32_split(__float_as_uint(b1[8 * j]), hi[j][1], lo[j][1]);
-            // kept in registers: loaded and split anew for every M tile otherwise
-            asm volatile("" : "+r"(hi[j][0]), "+r"(hi[j][1]), "+r"(lo[j][0]), "+r"(lo[j][1]));
-        }
+        for (int j = 0; j < NT; j++)
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                uint32_t x[3];
+                split_pair<3>(__float_as_uint((q ? lo1 : lo0)[8 * j]), __float_as_uint((q ? hi1 : hi0)[8 * j]), x);
+                // kept in registers: loaded and split anew for every M tile otherwise
+                asm volatile("" : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]));
+#pragma unroll
+                for (int i = 0; i < 3; i++) p[i][j][q] = x[i];
+            }
     }
 };
 
-// The split of an infinity or a NaN is not one (inf - inf), nor is that of a value which
-// rounds to infinity.  The kernels that write vectors set a flag where one is at or above
-// TF32_MAX (wide[0]: X, wide[1]: t), and the kernels launched after them, which read these
-// vectors, then multiply with FP32 multiply-adds (step_fma).  No kernel reads a flag that it
-// sets: its warps would disagree.
-__device__ __forceinline__ bool splits(float v) { return fabsf(v) < __uint_as_float(TF32_MAX_BITS); }
+// What the MMAs multiply must split and must not overflow on the way: an infinity or a NaN
+// does neither (inf - inf), nor does a part below BF16's range hold its bits.  The kernels
+// that write vectors record their range: range[j] the largest magnitude of vector j of X (the
+// bits of an FP32 value), range[RANGE_T] whether an entry of t is too large.  The kernels
+// launched after them, which read these vectors, multiply with FP32 multiply-adds instead
+// (step_fma) where a vector lies outside.  No kernel reads what it records itself: its warps
+// would disagree.  Within the range, sums of 512 products of a stored value below 2^59 and a
+// vector's entry below 2^59 are finite; a vector's entries are exact to 2^-63 of 2^-70.
+static constexpr unsigned RANGE_LARGE = (127u + 59) << 23;
+static constexpr unsigned RANGE_SMALL = (127u - 70) << 23;
+static constexpr int RANGE_T = 32;
+static_assert(MULTI_RANGE_WORDS == RANGE_T + 1, "the record's words");
+__device__ __forceinline__ bool too_large(float v) { return (__float_as_uint(v) & 0x7fffffffu) >= RANGE_LARGE; }
+// the same in every warp
+__device__ __forceinline__ bool out_of_range(const unsigned* range, int R)
+{
+    const int lane = threadIdx.x & 31;
+    const unsigned top = lane < R ? range[lane] : 0u;
+    return __any_sync(0xffffffffu, top >= RANGE_LARGE || (top != 0u && top < RANGE_SMALL));
+}
 
-// acc[j] += A B_j for one K step: FP32 values (three MMAs) or values that are TF32 (two)
-template <int NT, bool EXACT>
-__device__ __forceinline__ void step_mma(float (&acc)[NT][4], const uint32_t (&a)[4], const FragB<NT>& b)
+// acc[j] += A B_j for one step: A cut into three parts (FP32: nine MMAs), two (FP16: six) or
+// one (FP8: three)
+template <int NT, int PARTS>
+__device__ __forceinline__ void step_mma(float (&acc)[NT][4], const uint32_t (&a0)[4], const uint32_t (&a1)[4],
+                                         const FragB<NT>& b)
 {
     const float zero[4] = {0.f, 0.f, 0.f, 0.f};
-    if constexpr (EXACT) {
+    uint32_t a[PARTS][4];
 #pragma unroll
-        for (int j = 0; j < NT; j++) {
-            float d[4];
-            mma_tf32(d, a, b.lo[j], zero);
-            mma_tf32(d, a, b.hi[j], d);
-            add4(acc[j], d);
+    for (int q = 0; q < 4; q++) {
+        uint32_t x[PARTS];
+        split_pair<PARTS>(a0[q], a1[q], x);
+#pragma unroll
+        for (int i = 0; i < PARTS; i++) a[i][q] = x[i];
+    }
+#pragma unroll
+    for (int j = 0; j < NT; j++) {
+        float e[4], d[4], r[4];
+        mma_bf16(e, a[0], b.p[0][j], zero);
+        if constexpr (PARTS == 3) {
+            mma_bf16(d, a[2], b.p[1][j], zero);
+            mma_bf16(d, a[2], b.p[0][j], d);
+            mma_bf16(d, a[1], b.p[1][j], d);
+            mma_bf16(d, a[1], b.p[0][j], d);
+            const float n[4] = {-e[0], -e[1], -e[2], -e[3]};
+            mma_bf16(r, a[0], b.p[0][j], n);
+            mma_bf16(r, a[1], b.p[2][j], r);
+            mma_bf16(r, a[0], b.p[2][j], r);
+            mma_bf16(r, a[0], b.p[1][j], r);
+            add4(d, r);
+        } else if constexpr (PARTS == 2) {
+            mma_bf16(d, a[1], b.p[2][j], zero);
+            mma_bf16(d, a[1], b.p[1][j], d);
+            mma_bf16(d, a[0], b.p[2][j], d);
+            mma_bf16(d, a[1], b.p[0][j], d);
+            mma_bf16(d, a[0], b.p[1][j], d);
+        } else {
+            mma_bf16(d, a[0], b.p[2][j], zero);
+            mma_bf16(d, a[0], b.p[1][j], d);
         }
-    } else {
-        uint32_t ah[4], al[4];
-#pragma unroll
-        for (int q = 0; q < 4; q++) tf32_split(a[q], ah[q], al[q]);
-#pragma unroll
-        for (int j = 0; j < NT; j++) {
-            float d[4];
-            mma_tf32(d, al, b.hi[j], zero);
-            mma_tf32(d, ah, b.lo[j], d);
-            mma_tf32(d, ah, b.hi[j], d);
-            add4(acc[j], d);
-        }
+        add4(d, e);
+        add4(acc[j], d);
     }
 }
 
-// The same K step with FP32 multiply-adds: A from the warp's fragments, B row kk (slot
-// order) at b(kk).
+// Half of the step (8 K slots) with FP32 multiply-adds: A from the warp's fragments, B row
+// kk (slot order) at b(kk).
 template <int NT, class F>
 __device__ __forceinline__ void step_fma(float (&acc)[NT][4], const uint32_t (&a)[4], F b)
 {
@@ -180,15 +223,24 @@ __device__ __forceinline__ float2 e4m3x2_to_float2(uint32_t w)
     return __half22float2(*reinterpret_cast<const __half2*>(&h));
 }
 
-// X (caller order, column-major, FP64) as R FP32 values per point in Z order
-__global__ void k_gather_tf32(const double* X, int ldx, int nrhs, const int* perm2, int n, int R, float* xm, int* wide)
+// X (caller order, column-major, FP64) as R FP32 values per point in Z order, and the
+// vectors' largest magnitudes (256 threads a CTA)
+__global__ void k_gather_mma(const double* X, int ldx, int nrhs, const int* perm2, int n, int R, float* xm, unsigned* range)
 {
+    __shared__ unsigned top[32];
+    if (threadIdx.x < 32) top[threadIdx.x] = 0u;
+    __syncthreads();
     const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (idx >= (long long)n * R) return;
-    const int i = (int)(idx / R), j = (int)(idx - (long long)i * R);
-    const float v = j < nrhs ? (float)X[perm2[i] + (size_t)j * ldx] : 0.0f;
-    if (!splits(v)) *wide = 1;
-    xm[idx] = v;
+    if (idx < (long long)n * R) {
+        const int i = (int)(idx / R), j = (int)(idx - (long long)i * R);
+        const float v = j < nrhs ? (float)X[perm2[i] + (size_t)j * ldx] : 0.0f;
+        xm[idx] = v;
+        atomicMax(&top[j], __float_as_uint(v) & 0x7fffffffu);
+    }
+    __syncthreads();
+    // (read first: after a few CTAs hardly any has a larger one)
+    if (threadIdx.x < R && top[threadIdx.x] > *static_cast<volatile unsigned*>(range + threadIdx.x))
+        atomicMax(range + threadIdx.x, top[threadIdx.x]);
 }
 
 // ---------------------------------------------------------------------------
@@ -224,16 +276,16 @@ template <int NT> struct VtShape {
     static constexpr int SMEM = WARPS * (NS * STAGE + PART);
 };
 
-// t_b = V_b^T X_b, scaled.  M = 16 terms, N = 8 vectors, K = 8 columns of each MMA; a step
-// is 16 columns.  A lane's 16 bytes are columns 4t .. 4t+3 of a row: columns 4t, 4t+1 are
-// its K slots t, t+4 of the step's first MMA and 4t+2, 4t+3 of the second.  An FP16 row
+// t_b = V_b^T X_b, scaled.  M = 16 terms, N = 8 vectors, K = 16 columns of each MMA, a step.
+// A lane's 16 bytes are columns 4t .. 4t+3 of a row: columns 4t, 4t+1 are its K slots t, t+4
+// of the first half of the step and 4t+2, 4t+3 of the second.  An FP16 row
 // gives terms 2g, 2g+1 (M slots g, g+8); an FP8 row is read by two lane groups, each
 // taking two of its four terms.  Copies run ahead across tasks in a ring per warp, each
 // lane reading back what it copied (only X is shared by the warp).
 template <int NT>
 __global__ void __launch_bounds__(VtShape<NT>::WARPS * 32, 1)
-k_vtx_tf32(const VtTask* __restrict__ tasks, int nlarge, int nsmall, const float* __restrict__ xm,
-           float* __restrict__ tm, int* wide)
+k_vtx_mma(const VtTask* __restrict__ tasks, int nlarge, int nsmall, const float* __restrict__ xm,
+           float* __restrict__ tm, unsigned* range)
 {
     typedef VtShape<NT> S;
     constexpr int R = S::R, NS = S::NS, WARPS = S::WARPS;
@@ -261,9 +313,8 @@ k_vtx_tf32(const VtTask* __restrict__ tasks, int nlarge, int nsmall, const float
         }
     };
     const int ntask = nlarge + nsmall;
-    const bool plain = wide[0] != 0;
-    const double untruncate = plain ? 1.0 : UNTRUNCATE;
-    bool fits = true;
+    const bool plain = out_of_range(range, R);
+    bool large = false;
 
     // producer: the lane's rows of the task (offsets from the block's V, which may pass 4 GiB,
     // a bit per row that exists), its X rows, and the step
@@ -361,10 +412,9 @@ k_vtx_tf32(const VtTask* __restrict__ tasks, int nlarge, int nsmall, const float
             __syncwarp();
             const char* sa = ring + cslot + lane * 16;
             const float* sb = reinterpret_cast<const float*>(ring + cslot + VT_LD * 512);
-            FragB<NT> b[2];
+            FragB<NT> b;
             const float* bp = sb + 4 * lt * R + lt * 8 + lg;
-            b[0].get(bp, bp + R);
-            b[1].get(bp + 2 * R, bp + 3 * R);
+            b.get(bp, bp + R, bp + 2 * R, bp + 3 * R);
 #pragma unroll
             for (int m = 0; m < VT_MT; m++) {
                 if (m >= c.cnt) break;
@@ -375,10 +425,7 @@ k_vtx_tf32(const VtTask* __restrict__ tasks, int nlarge, int nsmall, const float
                     const uint4 w1 = *reinterpret_cast<const uint4*>(sm + 512);
                     a[0][0] = w0.x; a[0][1] = w1.x; a[0][2] = w0.y; a[0][3] = w1.y;
                     a[1][0] = w0.z; a[1][1] = w1.z; a[1][2] = w0.w; a[1][3] = w1.w;
-                    if constexpr (!PLAIN) {
-                        step_mma<NT, false>(acc[m], a[0], b[0]);
-                        step_mma<NT, false>(acc[m], a[1], b[1]);
-                    }
+                    if constexpr (!PLAIN) step_mma<NT, 3>(acc[m], a[0], a[1], b);
                 } else {
                     const uint32_t w[4] = {w0.x, w0.y, w0.z, w0.w};
                     const bool h16 = m < c16;
@@ -389,8 +436,8 @@ k_vtx_tf32(const VtTask* __restrict__ tasks, int nlarge, int nsmall, const float
                         a[q >> 1][2 * (q & 1) + 1] = __float_as_uint(f.y);
                     }
                     if constexpr (!PLAIN) {
-                        step_mma<NT, true>(acc[m], a[0], b[0]);
-                        step_mma<NT, true>(acc[m], a[1], b[1]);
+                        if (h16) step_mma<NT, 2>(acc[m], a[0], a[1], b);
+                        else step_mma<NT, 1>(acc[m], a[0], a[1], b);
                     }
                 }
                 if constexpr (PLAIN)
@@ -444,10 +491,11 @@ k_vtx_tf32(const VtTask* __restrict__ tasks, int nlarge, int nsmall, const float
                         }
                         const int term = m < c.cnt ? term_of(m, half) : -1;
                         if (term >= 0) {
-                            const double sc = (c.scal ? (double)c.scal[term] : 1.0) * untruncate;
-                            s.x = (float)(s.x * sc);
-                            s.y = (float)(s.y * sc);
-                            fits = fits && splits(s.x) && splits(s.y);
+                            if (c.scal) {
+                                s.x *= c.scal[term];
+                                s.y *= c.scal[term];
+                            }
+                            large = large || too_large(s.x) || too_large(s.y);
                             *reinterpret_cast<float2*>(tm + (size_t)(c.tout + term) * R + 8 * j + 2 * lt) = s;
                         }
                     }
@@ -459,11 +507,11 @@ k_vtx_tf32(const VtTask* __restrict__ tasks, int nlarge, int nsmall, const float
                 for (int half = 0; half < 2; half++) {
                     const int term = m < c.cnt ? term_of(m, half) : -1;
                     if (term < 0) continue;
-                    const double sc = (c.scal ? (double)c.scal[term] : 1.0) * untruncate;
+                    const float sc = c.scal ? c.scal[term] : 1.0f;
 #pragma unroll
                     for (int j = 0; j < NT; j++) {
-                        const float2 s = make_float2((float)(acc[m][j][2 * half] * sc), (float)(acc[m][j][2 * half + 1] * sc));
-                        fits = fits && splits(s.x) && splits(s.y);
+                        const float2 s = make_float2(acc[m][j][2 * half] * sc, acc[m][j][2 * half + 1] * sc);
+                        large = large || too_large(s.x) || too_large(s.y);
                         *reinterpret_cast<float2*>(tm + (size_t)(c.tout + term) * R + 8 * j + 2 * lt) = s;
                     }
                 }
@@ -479,7 +527,7 @@ k_vtx_tf32(const VtTask* __restrict__ tasks, int nlarge, int nsmall, const float
     if (plain) run(std::true_type{});
     else run(std::false_type{});
     cp_wait<0>();
-    if (!fits) wide[1] = 1;
+    if (large) range[RANGE_T] = 1u;
 }
 
 struct VtItem {
@@ -568,11 +616,11 @@ static hmg_status ensure_vt(hmg_matrix* h)
 // ---------------------------------------------------------------------------
 template <int NT> struct TtShape {
     static constexpr int R = 8 * NT;
-    // Warps a CTA: 12 are a multiple of a tile's 1 to 4 row groups, so that none is without
-    // work (24 vectors: 2.49 ms against 2.9 with 8 at 2^16 points, mixed); 8 where 12 would
-    // leave too few registers a thread (32 vectors: 6.9 ms against 7.35 at 2^17) or one CTA
-    // instead of two (16 vectors: 3.9 ms against 4.15).
-    static constexpr int WARPS = NT % 2 ? 12 : 8;
+    // Warps a CTA: 8 leave the registers that the fragments of all parts take (at 2^17 points,
+    // mixed: 8 vectors 3.42 ms against 4.30 with 12, 16 5.10 against 6.60, 32 8.41 against
+    // 9.72); with 24 vectors 12, a multiple of a tile's 1 to 4 row groups, so that none is
+    // without work (6.34 against 6.67; smaller tiles 3-4 % the other way).
+    static constexpr int WARPS = NT == 3 ? 12 : 8;
     static constexpr int SB = NT % 2 ? R : R + 8;        // floats between vector rows: lanes (g, t) hit 32 banks
     static constexpr int NS = NT <= 2 ? 3 : 4;           // stages a warp
     static constexpr int CTAS = NT <= 2 ? 2 : 1;
@@ -584,15 +632,15 @@ template <int NT> struct TtShape {
 };
 
 // One CTA per row tile, a warp per 32 rows and group of the tile's pairs.  M = 16 rows,
-// N = 8 vectors, K = 8 columns or terms of each MMA.  A lane's 16 bytes are 4 rows of a
+// N = 8 vectors, K = 16 columns or terms of each MMA.  A lane's 16 bytes are 4 rows of a
 // chunk column, the A rows g, g + 8 of two M tiles.  A stage is 16 terms of one tier (16
-// FP32, 8 FP16 pair or 4 FP8 quad columns: two K steps) and the vector rows they multiply,
+// FP32, 8 FP16 pair or 4 FP8 quad columns: one step) and the vector rows they multiply,
 // put in slot order.  Copies run NS - 1 stages ahead, across pairs.
 template <int NT>
 __global__ void __launch_bounds__(TtShape<NT>::WARPS * 32, TtShape<NT>::CTAS)
-k_tile_tf32(const PairDesc* __restrict__ desc, const int* tile_pair_start, const int* tile_r0, const int* tile_s,
+k_tile_mma(const PairDesc* __restrict__ desc, const int* tile_pair_start, const int* tile_r0, const int* tile_s,
             const int* perm1, const float* __restrict__ xm, const float* __restrict__ tm, const char* tbase, int nrhs,
-            double* Y, int ldy, int only_kind, const int* wide)
+            double* Y, int ldy, int only_kind, const unsigned* range)
 {
     typedef TtShape<NT> S;
     constexpr int R = S::R, NS = S::NS, SB = S::SB;
@@ -606,8 +654,7 @@ k_tile_tf32(const PairDesc* __restrict__ desc, const int* tile_pair_start, const
     char* ring = tt_smem + (size_t)warp * NS * S::STAGE;
     const uint32_t ring_s = static_cast<uint32_t>(__cvta_generic_to_shared(ring));
     const int pend = g < G ? tile_pair_start[t + 1] : 0;
-    const bool plain = (wide[0] | wide[1]) != 0;
-    const double untruncate = plain ? 1.0 : UNTRUNCATE;
+    const bool plain = out_of_range(range, R) || range[RANGE_T] != 0u;
 
     // producer: pair; within it the tier (0 FP32, 1 FP16, 2 FP8), the lane's next slice and
     // vector addresses, chunk columns left in the tier
@@ -674,7 +721,7 @@ k_tile_tf32(const PairDesc* __restrict__ desc, const int* tile_pair_start, const
             for (int i = 0; i < NT; i++)
                 cp_vector16(ring_s + pslot + wdst[i], wp + wrow(i) * R + wc4(i), wrow(i) < terms);
             // the next stage of the tier, of the pair's next tier, or of the next pair
-            int hdr = kind | (kind < 2 && terms <= 8 ? 8 : 0);  // one K step (FP8 terms lie in both)
+            int hdr = kind;
             ap += (size_t)(used * sp) * 4;
             wp += (used << kind) * R;
             left -= used;
@@ -716,7 +763,7 @@ k_tile_tf32(const PairDesc* __restrict__ desc, const int* tile_pair_start, const
         const int hdr = *reinterpret_cast<const int*>(st + S::STAGE - 16);
         const int k = hdr & 3;
         const float* bp = reinterpret_cast<const float*>(st + S::VOFF);
-        // the A fragments of K step i for the two M tiles
+        // the A fragments of half i of the step for the two M tiles
         auto frag = [&](int i, uint32_t (&a0)[4], uint32_t (&a1)[4]) {
             if (k == 0) {
                 const uint4 w0 = *reinterpret_cast<const uint4*>(sa + (2 * i) * 512);
@@ -741,36 +788,21 @@ k_tile_tf32(const PairDesc* __restrict__ desc, const int* tile_pair_start, const
             a1[2] = __float_as_uint(f2.y); a1[3] = __float_as_uint(f3.y);
         };
         if constexpr (!PLAIN) {
-            // few vectors: both K steps at once (an empty one multiplies zeros), so that
-            // their loads and MMAs overlap; many: one at a time, empty ones left out
-            constexpr int KS = NT <= 2 ? 2 : 1;
-#pragma unroll
-            for (int i0 = 0; i0 < 2; i0 += KS) {
-                if (i0 == 1 && (hdr & 8)) break;
-                FragB<NT> b[KS];
-#pragma unroll
-                for (int i = 0; i < KS; i++)
-                    b[i].get(bp + (8 * (i0 + i) + lt) * SB + lg, bp + (8 * (i0 + i) + 4 + lt) * SB + lg);
-                if (k == 0) {
-#pragma unroll
-                    for (int i = 0; i < KS; i++) {
-                        uint32_t a0[4], a1[4];
-                        const uint4 w0 = *reinterpret_cast<const uint4*>(sa + (2 * (i0 + i)) * 512);
-                        const uint4 w1 = *reinterpret_cast<const uint4*>(sa + (2 * (i0 + i) + 1) * 512);
-                        a0[0] = w0.x; a0[1] = w0.y; a0[2] = w1.x; a0[3] = w1.y;
-                        a1[0] = w0.z; a1[1] = w0.w; a1[2] = w1.z; a1[3] = w1.w;
-                        step_mma<NT, false>(acc[0], a0, b[i]);
-                        step_mma<NT, false>(acc[1], a1, b[i]);
-                    }
-                } else {
-#pragma unroll
-                    for (int i = 0; i < KS; i++) {
-                        uint32_t a0[4], a1[4];
-                        frag(i0 + i, a0, a1);
-                        step_mma<NT, true>(acc[0], a0, b[i]);
-                        step_mma<NT, true>(acc[1], a1, b[i]);
-                    }
-                }
+            FragB<NT> b;
+            const float* br = bp + lt * SB + lg;
+            b.get(br, br + 4 * SB, br + 8 * SB, br + 12 * SB);
+            uint32_t a0[2][4], a1[2][4];
+            frag(0, a0[0], a1[0]);
+            frag(1, a0[1], a1[1]);
+            if (k == 0) {
+                step_mma<NT, 3>(acc[0], a0[0], a0[1], b);
+                step_mma<NT, 3>(acc[1], a1[0], a1[1], b);
+            } else if (k == 1) {
+                step_mma<NT, 2>(acc[0], a0[0], a0[1], b);
+                step_mma<NT, 2>(acc[1], a1[0], a1[1], b);
+            } else {
+                step_mma<NT, 1>(acc[0], a0[0], a0[1], b);
+                step_mma<NT, 1>(acc[1], a1[0], a1[1], b);
             }
         } else {
 #pragma unroll
@@ -787,7 +819,7 @@ k_tile_tf32(const PairDesc* __restrict__ desc, const int* tile_pair_start, const
 #pragma unroll
                 for (int j = 0; j < NT; j++)
 #pragma unroll
-                    for (int q = 0; q < 4; q++) acc64[m][j][q] = fma((double)acc[m][j][q], untruncate, acc64[m][j][q]), acc[m][j][q] = 0.0f;
+                    for (int q = 0; q < 4; q++) acc64[m][j][q] += acc[m][j][q], acc[m][j][q] = 0.0f;
         }
         cslot = cslot + S::STAGE == NS * S::STAGE ? 0u : cslot + S::STAGE;
         __syncwarp();  // the slot is refilled next
@@ -837,32 +869,32 @@ k_tile_tf32(const PairDesc* __restrict__ desc, const int* tile_pair_start, const
 
 template <int NT>
 static hmg_status launch_tiles(hmg_matrix* h, const float* xm, const float* tm, int nrhs, double* Y, int ldy,
-                               int only_kind, const int* wide)
+                               int only_kind, const unsigned* range)
 {
     if (h->ntiles <= 0) return HMG_OK;
-    HMG_CUDA_TRY(cudaFuncSetAttribute(k_tile_tf32<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, TtShape<NT>::SMEM));
-    k_tile_tf32<NT><<<h->ntiles, TtShape<NT>::WARPS * 32, TtShape<NT>::SMEM, h->stream>>>(
+    HMG_CUDA_TRY(cudaFuncSetAttribute(k_tile_mma<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, TtShape<NT>::SMEM));
+    k_tile_mma<NT><<<h->ntiles, TtShape<NT>::WARPS * 32, TtShape<NT>::SMEM, h->stream>>>(
         static_cast<const PairDesc*>(h->tile_desc), h->tile_desc_start, h->tile_r0, h->tile_s, h->perm[0], xm, tm,
-        static_cast<const char*>(h->tbuf), nrhs, Y, ldy, only_kind, wide);
+        static_cast<const char*>(h->tbuf), nrhs, Y, ldy, only_kind, range);
     HMG_LAUNCH_CHECK();
     return HMG_OK;
 }
 
 template <int NT>
-static hmg_status launch_all(hmg_matrix* h, const float* xm, float* tm, int nrhs, double* Y, int ldy, int* wide)
+static hmg_status launch_all(hmg_matrix* h, const float* xm, float* tm, int nrhs, double* Y, int ldy, unsigned* range)
 {
     const int nl = h->vt_large, ns = h->vt_small;
     if (nl + ns > 0) {
-        HMG_CUDA_TRY(cudaFuncSetAttribute(k_vtx_tf32<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, VtShape<NT>::SMEM));
+        HMG_CUDA_TRY(cudaFuncSetAttribute(k_vtx_mma<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, VtShape<NT>::SMEM));
         const int grid = std::min(h->nsm, nl + ceil_div(ns, VtShape<NT>::WARPS));
-        k_vtx_tf32<NT><<<grid, VtShape<NT>::WARPS * 32, VtShape<NT>::SMEM, h->stream>>>(static_cast<const VtTask*>(h->vt_tasks), nl,
-                                                                              ns, xm, tm, wide);
+        k_vtx_mma<NT><<<grid, VtShape<NT>::WARPS * 32, VtShape<NT>::SMEM, h->stream>>>(static_cast<const VtTask*>(h->vt_tasks), nl,
+                                                                              ns, xm, tm, range);
         HMG_LAUNCH_CHECK();
     }
-    return launch_tiles<NT>(h, xm, tm, nrhs, Y, ldy, -1, wide);
+    return launch_tiles<NT>(h, xm, tm, nrhs, Y, ldy, -1, range);
 }
 
-hmg_status matvec_multi_tf32(hmg_matrix* h, int nrhs, const double* X, int ldx, double* Y, int ldy)
+hmg_status matvec_multi_mma(hmg_matrix* h, int nrhs, const double* X, int ldx, double* Y, int ldy)
 {
     cudaStream_t s = h->stream;
     hmg_status st;
@@ -870,15 +902,15 @@ hmg_status matvec_multi_tf32(hmg_matrix* h, int nrhs, const double* X, int ldx, 
     if ((st = ensure_desc(h, 4)) || (st = ensure_vt(h))) return st;
     float* xm = nullptr;
     float* tm = nullptr;
-    // the flags of values the split does not take sit behind xm
-    if ((st = dalloc(&xm, (size_t)h->n[1] * R + 2, s)) || (st = dalloc(&tm, (size_t)(h->rank_total + 1) * R, s))) {
+    // the range record sits behind xm
+    if ((st = dalloc(&xm, (size_t)h->n[1] * R + MULTI_RANGE_WORDS, s)) || (st = dalloc(&tm, (size_t)(h->rank_total + 1) * R, s))) {
         dfree(xm, s);
         return st;
     }
-    int* wide = reinterpret_cast<int*>(xm + (size_t)h->n[1] * R);
-    cudaError_t e = cudaMemsetAsync(wide, 0, 2 * sizeof(int), s);
+    unsigned* range = reinterpret_cast<unsigned*>(xm + (size_t)h->n[1] * R);
+    cudaError_t e = cudaMemsetAsync(range, 0, MULTI_RANGE_WORDS * sizeof(unsigned), s);
     if (e == cudaSuccess) {
-        k_gather_tf32<<<ceil_div((long long)h->n[1] * R, 256), 256, 0, s>>>(X, ldx, nrhs, h->perm[1], h->n[1], R, xm, wide);
+        k_gather_mma<<<ceil_div((long long)h->n[1] * R, 256), 256, 0, s>>>(X, ldx, nrhs, h->perm[1], h->n[1], R, xm, range);
         e = cudaGetLastError();
     }
     if (e != cudaSuccess) {
@@ -886,10 +918,10 @@ hmg_status matvec_multi_tf32(hmg_matrix* h, int nrhs, const double* X, int ldx, 
         st = HMG_ERR_CUDA;
     } else {
         switch (nt) {
-        case 1: st = launch_all<1>(h, xm, tm, nrhs, Y, ldy, wide); break;
-        case 2: st = launch_all<2>(h, xm, tm, nrhs, Y, ldy, wide); break;
-        case 3: st = launch_all<3>(h, xm, tm, nrhs, Y, ldy, wide); break;
-        default: st = launch_all<4>(h, xm, tm, nrhs, Y, ldy, wide); break;
+        case 1: st = launch_all<1>(h, xm, tm, nrhs, Y, ldy, range); break;
+        case 2: st = launch_all<2>(h, xm, tm, nrhs, Y, ldy, range); break;
+        case 3: st = launch_all<3>(h, xm, tm, nrhs, Y, ldy, range); break;
+        default: st = launch_all<4>(h, xm, tm, nrhs, Y, ldy, range); break;
         }
     }
     dfree(xm, s);
@@ -898,19 +930,19 @@ hmg_status matvec_multi_tf32(hmg_matrix* h, int nrhs, const double* X, int ldx, 
 }
 
 // Y = the near-field part of H X for up to 32 vectors, FP32 stored near field (the BF16
-// tensor-core path with its near field in FP32).  xm: n2 x 32 values and two flags.
+// tensor-core path with its near field in FP32).  xm: n2 x 32 values and the range record.
 hmg_status near_multi32(hmg_matrix* h, const double* X, int ldx, int nrhs, float* xm, double* Y, int ldy)
 {
     // a product in another near-field mode or arithmetic may have left other descriptors, and
     // one that ran out of memory none
     hmg_status st = ensure_desc(h, 4);
     if (st) return st;
-    int* wide = reinterpret_cast<int*>(xm + (size_t)h->n[1] * 32);
-    HMG_CUDA_TRY(cudaMemsetAsync(wide, 0, 2 * sizeof(int), h->stream));
-    k_gather_tf32<<<ceil_div((long long)h->n[1] * 32, 256), 256, 0, h->stream>>>(X, ldx, nrhs, h->perm[1], h->n[1], 32,
-                                                                                xm, wide);
+    unsigned* range = reinterpret_cast<unsigned*>(xm + (size_t)h->n[1] * 32);
+    HMG_CUDA_TRY(cudaMemsetAsync(range, 0, MULTI_RANGE_WORDS * sizeof(unsigned), h->stream));
+    k_gather_mma<<<ceil_div((long long)h->n[1] * 32, 256), 256, 0, h->stream>>>(X, ldx, nrhs, h->perm[1], h->n[1], 32,
+                                                                                xm, range);
     HMG_LAUNCH_CHECK();
-    return launch_tiles<4>(h, xm, nullptr, nrhs, Y, ldy, PAIR_STORED, wide);
+    return launch_tiles<4>(h, xm, nullptr, nrhs, Y, ldy, PAIR_STORED, range);
 }
 
 }  // namespace hmg

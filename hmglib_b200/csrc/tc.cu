@@ -955,7 +955,7 @@ static hmg_status tc_product(hmg_matrix* h, int nrhs, const double* X, int ldx, 
     if (!h->tc_near && h->ndense > 0) {
         // the near field in FP32 writes every row of Y first (32 vectors a pass)
         float* xm = nullptr;
-        if ((st = dalloc(&xm, (size_t)h->n[1] * 32 + 2, s))) return st;
+        if ((st = dalloc(&xm, (size_t)h->n[1] * 32 + MULTI_RANGE_WORDS, s))) return st;
         for (int j0 = 0; j0 < nrhs && !st; j0 += 32)
             st = near_multi32(h, X + (size_t)j0 * ldx, ldx, std::min(32, nrhs - j0), xm, Y + (size_t)j0 * ldy, ldy);
         dfree(xm, s);
