@@ -910,6 +910,7 @@ void free_far(hmg_matrix* h)
     dfree(h->far_list, s);
     dfree(h->vt_tasks, s);
     h->vt_large = h->vt_small = 0;
+    h->stored_range = -1;
     dfree(h->tier32, s);
     dfree(h->tier16, s);
     h->h_r32.clear();

@@ -133,6 +133,7 @@ struct hmg_matrix {
     int k1_task_start[3][5] = {};   // per tier: first warp task of each class, task count
     void* vt_tasks = nullptr;      // multi-vector V^T X tasks (multi_mma.cu), the split ones first
     int vt_large = 0, vt_small = 0;
+    int stored_range = -1;         // FP32 values within the MMAs' range (multi_mma.cu): 1, outside: 0, not looked at: -1
     int* far_list = nullptr;       // admissible blocks with rank > 0 (streaming V^T x)
     int nfar_list = 0;
     int* dev_err = nullptr;        // pipeline wait time-out flag (0 = fine)

@@ -62,6 +62,7 @@ void free_near(hmg_matrix* h)
     dfree(h->near_off, h->stream);
     h->near_prec = -1;
     h->near_stored = 0;
+    h->stored_range = -1;
     h->desc_near_mode = -1;
     if (h->near_mode == HMG_NEAR_STORED) h->near_mode = HMG_NEAR_ONTHEFLY;
     free_tc(h);  // its BF16 near slices are copies of this storage

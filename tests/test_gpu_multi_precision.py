@@ -87,3 +87,41 @@ def test_both_ends_of_the_range(hmg, cuda, storage, log2):
     for j in range(5):
         assert rel_err(B[j].cpu().numpy(), A[j].cpu().numpy()) < 1e-6
     H.close()
+
+
+@pytest.mark.parametrize("reg", [3.39e38, 1e39, -1e39, 1e13])
+@pytest.mark.parametrize("storage", ["fp32", "mixed"])
+def test_stored_values_that_do_not_split(hmg, cuda, storage, reg):
+    """A regularization near, beyond and far below the FP32 limit: the stored diagonal is huge or
+    infinite, and the multi-vector products have the single-vector product's finite, infinite
+    and undefined entries (one vector is zero at some points) and its values to 1e-6."""
+    torch = cuda
+    n = 3000
+    p = make_points("uniform", n, 2, 5)
+    H = engine(hmg, p, p, 1.5, 64, rule=1)
+    H.set_kernel(GAUSS, 0.05, reg)
+    H.precompute_aca(64, 1e-8, hmg.PREC_MIXED if storage == "mixed" else hmg.PREC_FP32)
+    H.precompute_dense(hmg.PREC_FP32)
+    X = torch.from_numpy(np.random.default_rng(1).uniform(0.1, 0.9, (3, n))).cuda()
+    X[1, ::7] = 0.0
+    X[2] *= -1.0
+    Y, y = torch.empty_like(X), torch.empty(n, dtype=torch.float64, device="cuda")
+    H.matvec_multi(X, Y)
+    for j in range(3):
+        H.matvec(X[j], y)
+        torch.cuda.synchronize()
+        a, one = Y[j].cpu().numpy(), y.cpu().numpy()
+        np.testing.assert_array_equal(np.isfinite(a), np.isfinite(one))
+        np.testing.assert_array_equal(a[np.isinf(one)], one[np.isinf(one)])
+        fin = np.isfinite(one)
+        if fin.any():
+            assert rel_err(a[fin], one[fin]) < 1e-6
+    # another regularization, the same handle: back to finite products
+    H.set_kernel(GAUSS, 0.05, 0.5)
+    H.precompute_aca(64, 1e-8, hmg.PREC_MIXED if storage == "mixed" else hmg.PREC_FP32)
+    H.precompute_dense(hmg.PREC_FP32)
+    H.matvec_multi(X, Y)
+    H.matvec(X[0], y)
+    torch.cuda.synchronize()
+    assert rel_err(Y[0].cpu().numpy(), y.cpu().numpy()) < 1e-6
+    H.close()
