@@ -271,13 +271,14 @@ static constexpr int VT_SPLIT_COLS = 1024;
 
 template <int NT> struct VtShape {
     static constexpr int R = 8 * NT;
-    // warps a CTA: what shared memory holds of rings and partial sums (210, 205, 169, 190 KB)
+    // warps a CTA: what shared memory holds of rings and partial sums (206, 197, 159, 187 KB)
     static constexpr int WARPS = NT == 1 ? 16 : (NT == 2 ? 12 : 8);
     static constexpr int NS = 3;                                     // stages a warp
     static constexpr int BF = 16 * R + 32;                           // floats of a stage's 16 X rows
     static constexpr int STAGE = VT_LD * 512 + BF * 4;
     static constexpr int PART = VT_MT * 16 * R * 4;                  // one warp's partial sums
     static constexpr int SMEM = WARPS * (NS * STAGE + PART);
+    static_assert(SMEM <= 227 * 1024, "the shared memory of a CTA");
 };
 
 // t_b = V_b^T X_b, scaled.  M = 16 terms, N = 8 vectors, K = 16 columns of each MMA, a step.
@@ -708,8 +709,8 @@ k_tile_mma(const PairDesc* __restrict__ desc, const int* tile_pair_start, const 
     open_pair();
     int prod = 0;
     uint32_t pslot = 0;
-    // the lane's columns of a stage, or none where it has no rows
-    const int lta = row0 < sp ? lt : 64;
+    // the lane's columns of a stage, or none (beyond every pair's) where it has no rows
+    const int lta = row0 < sp ? lt : 1 << 20;
     auto issue = [&]() {
         if (left > 0) {
             const uint32_t sa = ring_s + pslot + lane * 16;

@@ -48,7 +48,7 @@ __device__ __forceinline__ uint4 ld_stream(const void* p)
         : "l"(p));
     return v;
 }
-// longest pair a tile kernel's warp takes whole (see free_tile_desc)
+// longest pair a tile kernel's warp takes whole (why: k_count_chunks in matvec.cu)
 static constexpr int TILE_CHUNK = 256;
 // largest rank the streaming V^T x kernel accepts
 static constexpr int K1_MAXRANK = 128;

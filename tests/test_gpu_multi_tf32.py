@@ -1,6 +1,6 @@
-"""Multi-vector products on TF32 tensor-core operands (FP32 and mixed storage, 2 to 32
+"""Multi-vector products on split tensor-core operands (FP32 and mixed storage, 2 to 32
 vectors a pass): accuracy against 64 bits at the edges of the kernels' tiles, and the
-values that the TF32 split does not take.  No reference counterpart (the reference
+values that the split does not take.  No reference counterpart (the reference
 multiplies one vector per apply_h_matrix_mvp call, hmglib.cu:271-286)."""
 import numpy as np
 import pytest
@@ -22,7 +22,7 @@ def _build(hmg, gen, n, dim, leaf, prec, eps=1e-8, kmax=96, rule=1):
 
 
 # Tolerance: FP32 entries, vectors and sums (2^-24 each, sums over up to 16384 columns in
-# chains of 8 per FP32 addition) and the ACA's and the short tiers' own error at eps 1e-8,
+# steps of 16 per FP32 addition) and the ACA's and the short tiers' own error at eps 1e-8,
 # 1e-7 each: below 1e-6 together, the bound the engine states for these products.
 @pytest.mark.parametrize("case", [
     ("uniform", 700, 2, 16),      # tiles of at most 16 rows, ranks below one K step
@@ -112,7 +112,7 @@ def test_sums_that_overflow_on_the_way(hmg, cuda, storage):
     X = torch.from_numpy(np.random.default_rng(3).uniform(-1, 1, (9, n))).cuda()
     Y0 = torch.empty_like(X)
     H.matvec_multi(X, Y0)
-    X[4] = 2e36  # finite, and so is its TF32 rounding; sums of 200 of them are not
+    X[4] = 2e36  # finite; sums of 200 of them are not
     Y, Z = torch.empty_like(X), torch.empty_like(X)
     H.matvec_multi(X, Y)
     for _ in range(20):
