@@ -40,6 +40,7 @@
 #include <vector>
 
 #include "hmg_matrix.cuh"
+#include "stream.cuh"
 
 namespace hmg {
 
@@ -713,7 +714,7 @@ static hmg_status launch_small(BlockGeom g, const KernelSpec& K, const PointsVie
 template <typename T>
 __global__ void __launch_bounds__(256) k_aca_compact(BlockGeom g, AcaBatch B, const int* tile_r0, const int* tile_s,
                                                      const int* tile_pstart, const int* tfirst, const int* tlast,
-                                                     T* const* ptrU, T* const* ptrV)
+                                                     T* const* ptrU, T* const* ptrV, unsigned* top)
 {
     const int e = blockIdx.x;
     const int b = B.blocks[e];
@@ -726,14 +727,27 @@ __global__ void __launch_bounds__(256) k_aca_compact(BlockGeom g, AcaBatch B, co
     T* dU = ptrU[b];
     T* dV = ptrV[b];
     const int m2p = (m2 + 3) & ~3;
+    unsigned top_u = 0u, top_v = 0u;
     for (int l = warp; l < r; l += 8)
-        for (int j = lane; j < m2p; j += 32) dV[(size_t)l * m2p + j] = j < m2 ? (T)V[j + (size_t)l * m2] : (T)0;
+        for (int j = lane; j < m2p; j += 32) {
+            const T v = j < m2 ? (T)V[j + (size_t)l * m2] : (T)0;
+            dV[(size_t)l * m2p + j] = v;
+            if constexpr (sizeof(T) == 4) top_v = max(top_v, magnitude(v));
+        }
     const int p0 = tile_pstart[tfirst[b]];
     for (int t = tfirst[b]; t <= tlast[b]; t++) {
         const int s = tile_s[t], sp = (s + 3) & ~3, tr = tile_r0[t] - r0;
         T* dst = dU + (size_t)(tile_pstart[t] - p0) * r;
         for (int l = warp; l < r; l += 8)
-            for (int i = lane; i < sp; i += 32) dst[(size_t)l * sp + i] = i < s ? (T)U[(size_t)l * m1 + tr + i] : (T)0;
+            for (int i = lane; i < sp; i += 32) {
+                const T u = i < s ? (T)U[(size_t)l * m1 + tr + i] : (T)0;
+                dst[(size_t)l * sp + i] = u;
+                if constexpr (sizeof(T) == 4) top_u = max(top_u, magnitude(u));
+            }
+    }
+    if constexpr (sizeof(T) == 4) {
+        record_top(top_u, top + 1);
+        record_top(top_v, top + 2);
     }
 }
 
@@ -819,7 +833,7 @@ __global__ void __launch_bounds__(256) k_aca_tiers(AcaBatch B, TierOut T, int ne
 __global__ void __launch_bounds__(256)
 k_aca_compact_mixed(BlockGeom g, AcaBatch B, TierOut T, const int* tile_r0, const int* tile_s,
                     const int* tile_pstart, const int* tfirst, const int* tlast, void* const* ptrU,
-                    void* const* ptrV)
+                    void* const* ptrV, unsigned* top)
 {
     const int e = blockIdx.x;
     const int b = B.blocks[e];
@@ -835,7 +849,8 @@ k_aca_compact_mixed(BlockGeom g, AcaBatch B, TierOut T, const int* tile_r0, cons
     // dst[0 .. rows): the storage words of a word column -- FP32, FP16 pairs or FP8 quads --
     // from term l0 on, rows n.. zero (src + l ld: term l; sc: the terms' scales).  Four
     // entries a lane at a time, so that their loads overlap.
-    auto convert = [&](uint32_t* dst, int rows, const double* src, size_t ld, int l0, int kind, int n, const float* sc) {
+    auto convert = [&](uint32_t* dst, int rows, const double* src, size_t ld, int l0, int kind, int n, const float* sc,
+                       unsigned& largest) {
         src += (size_t)l0 * ld;
         const int nt = 1 << kind;
         double q[4];
@@ -853,6 +868,7 @@ k_aca_compact_mixed(BlockGeom g, AcaBatch B, TierOut T, const int* tile_r0, cons
                 uint32_t w;
                 if (kind == 0) {
                     w = __float_as_uint((float)x[u][0]);
+                    largest = max(largest, w & 0x7fffffffu);
                 } else if (kind == 1) {
                     const __half2 h = __halves2half2(__float2half_rn((float)(x[u][0] / q[0])), __float2half_rn((float)(x[u][1] / q[1])));
                     w = *reinterpret_cast<const uint32_t*>(&h);
@@ -872,11 +888,12 @@ k_aca_compact_mixed(BlockGeom g, AcaBatch B, TierOut T, const int* tile_r0, cons
         l0 = kind == 0 ? c : (kind == 1 ? r32 + 2 * (c - r32) : r32 + r16 + 4 * (c - r32 - (r16 >> 1)));
     };
     const int nc = r32 + (r16 >> 1) + (r8 >> 2);
+    unsigned top_u = 0u, top_v = 0u;  // of the FP32 words
     uint32_t* vw = reinterpret_cast<uint32_t*>(ptrV[b]);
     for (int c = warp; c < nc; c += 8) {
         int kind, l0;
         column(c, kind, l0);
-        convert(vw + (size_t)c * m2p, m2p, V, m2, l0, kind, m2, T.sv + so);
+        convert(vw + (size_t)c * m2p, m2p, V, m2, l0, kind, m2, T.sv + so, top_v);
     }
     float* scal = reinterpret_cast<float*>(vw + (size_t)nc * m2p);
     for (int l = threadIdx.x; l < r; l += blockDim.x) scal[l] = T.su[so + l] * T.sv[so + l];
@@ -890,9 +907,11 @@ k_aca_compact_mixed(BlockGeom g, AcaBatch B, TierOut T, const int* tile_r0, cons
         for (int c = warp; c < nc; c += 8) {
             int kind, l0;
             column(c, kind, l0);
-            convert(slice + (size_t)c * sp, sp, U + tr, m1, l0, kind, s, T.su + so);
+            convert(slice + (size_t)c * sp, sp, U + tr, m1, l0, kind, s, T.su + so, top_u);
         }
     }
+    record_top(top_u, top + 1);
+    record_top(top_v, top + 2);
 }
 
 void free_far(hmg_matrix* h)
@@ -910,7 +929,6 @@ void free_far(hmg_matrix* h)
     dfree(h->far_list, s);
     dfree(h->vt_tasks, s);
     h->vt_large = h->vt_small = 0;
-    h->stored_range = -1;
     dfree(h->tier32, s);
     dfree(h->tier16, s);
     h->h_r32.clear();
@@ -928,8 +946,9 @@ void free_far(hmg_matrix* h)
 // run_aca returns, its kernels have ended and the scratch is given back.  The factors' part
 // is up to 4 GB, which the stream-ordered pool maps and unmaps at 6.3 ms a GB each way; a
 // cudaMalloc and its cudaFree take 0.7 ms and 0.8 more a GB (measured), so from 64 MB on it
-// comes from there.  (cudaFree waits for the device; products on another stream beside
-// builds of 131,072 points: p50 1.60 ms with pool scratch, 1.78 now, p99 115 and 36 ms.)
+// comes from there.  (cudaFree waits for the device.  Products of 1.53 ms on another stream,
+// beside one construction of 131,072 points after another: p99 115 ms with 16 GB of pool
+// scratch and the former kernels, 36 ms now.)
 struct AcaScratch {
     static constexpr size_t POOLED = (64u << 20) / sizeof(double);
     hmg_matrix* h;
@@ -1002,6 +1021,7 @@ hmg_status run_aca(hmg_matrix* h, int k, double eps, int precision)
         (st = dalloc((void***)&h->ptrV, (size_t)nb, s)) ||
         (st = dalloc(&h->tier32, (size_t)nb, s)) || (st = dalloc(&h->tier16, (size_t)nb, s)))
         return st;
+    HMG_CUDA_TRY(cudaMemsetAsync(h->stored_top + 1, 0, 2 * sizeof(unsigned), s));
 
     // batches of admissible blocks whose FP64 scratch fits the budget
     size_t free_b = 0, total_b = 0;
@@ -1189,15 +1209,15 @@ hmg_status run_aca(hmg_matrix* h, int k, double eps, int precision)
                                          cudaMemcpyHostToDevice, s));
             if (mixed)
                 k_aca_compact_mixed<<<ne, 256, 0, s>>>(g, B, T, h->tile_r0, h->tile_s, h->tile_pstart,
-                                                       h->blk_tfirst, h->blk_tlast, h->ptrU, h->ptrV);
+                                                       h->blk_tfirst, h->blk_tlast, h->ptrU, h->ptrV, h->stored_top);
             else if (precision == HMG_PREC_FP64)
                 k_aca_compact<double><<<ne, 256, 0, s>>>(g, B, h->tile_r0, h->tile_s, h->tile_pstart,
                                                          h->blk_tfirst, h->blk_tlast,
-                                                         (double* const*)h->ptrU, (double* const*)h->ptrV);
+                                                         (double* const*)h->ptrU, (double* const*)h->ptrV, nullptr);
             else
                 k_aca_compact<float><<<ne, 256, 0, s>>>(g, B, h->tile_r0, h->tile_s, h->tile_pstart,
                                                         h->blk_tfirst, h->blk_tlast,
-                                                        (float* const*)h->ptrU, (float* const*)h->ptrV);
+                                                        (float* const*)h->ptrU, (float* const*)h->ptrV, h->stored_top);
             HMG_LAUNCH_CHECK();
         }
         HMG_CUDA_TRY(cudaStreamSynchronize(s));

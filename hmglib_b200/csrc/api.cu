@@ -44,6 +44,7 @@ static void free_matrix_buffers(hmg_matrix* h)
     dfree(h->k1_units, s);
     dfree(h->far_list, s);
     dfree(h->dev_err, s);
+    dfree(h->stored_top, s);
     dfree(h->dev_x, s); dfree(h->dev_y, s);
 }
 
@@ -73,6 +74,8 @@ hmg_status hmg_create(hmg_matrix** out, int n1, int n2, int dim, int bits, void*
     h->pool_generation = pool_retain(h->device);
     hmg_status st = dalloc(&h->dev_err, 4, h->stream);  // [0] error flag, [1],[2] work counters
     if (!st && cudaMemsetAsync(h->dev_err, 0, 4 * sizeof(int), h->stream) != cudaSuccess) st = HMG_ERR_CUDA;
+    if (!st) st = dalloc(&h->stored_top, 3, h->stream);
+    if (!st && cudaMemsetAsync(h->stored_top, 0, 3 * sizeof(unsigned), h->stream) != cudaSuccess) st = HMG_ERR_CUDA;
     for (int i = 0; i < 2 && !st; i++) {
         size_t n = (size_t)h->n[i];
         if ((st = dalloc(&h->pts[i], n * dim, h->stream)) || (st = dalloc(&h->zpts[i], n * dim, h->stream)) ||

@@ -133,10 +133,10 @@ struct hmg_matrix {
     int k1_task_start[3][5] = {};   // per tier: first warp task of each class, task count
     void* vt_tasks = nullptr;      // multi-vector V^T X tasks (multi_mma.cu), the split ones first
     int vt_large = 0, vt_small = 0;
-    int stored_range = -1;         // FP32 values within the MMAs' range (multi_mma.cu): 1, outside: 0, not looked at: -1
     int* far_list = nullptr;       // admissible blocks with rank > 0 (streaming V^T x)
     int nfar_list = 0;
     int* dev_err = nullptr;        // pipeline wait time-out flag (0 = fine)
+    unsigned* stored_top = nullptr;  // largest magnitudes (bits) of the stored FP32 near field, U and V
     int matvec_variant = 1;        // 0: streaming kernels where applicable, 1: plain-load kernels
     int k1_piece_bytes = 65536;    // K1 warp-task unit: V^T rows of one tier up to these bytes (hmg_autotune)
     int k1_ctas_per_sm = 8;        // K1 grid: CTAs per SM (hmg_autotune)
@@ -168,6 +168,7 @@ hmg_status load(hmg_matrix** out, const char* path, cudaStream_t s);
 hmg_status run_aca(hmg_matrix* h, int k, double eps, int precision);
 hmg_status fill_near(hmg_matrix* h, int precision);
 hmg_status ensure_side_streams(hmg_matrix* h);
+hmg_status scan_stored_top(hmg_matrix* h);
 hmg_status matvec_device(hmg_matrix* h, const double* x, double* y, bool fp64_arith = false);
 hmg_status matvec_unbatched(hmg_matrix* h, const double* x, double* y);
 hmg_status matvec_multi(hmg_matrix* h, int nrhs, const double* X, int ldx, double* Y, int ldy);

@@ -522,6 +522,7 @@ static hmg_status upload(hmg_matrix* h, Reader& R, const Header& H, const Plan& 
         h->near_stored = H.near_stored;
     }
     h->near_mode = H.near_mode;
+    if ((st = scan_stored_top(h))) return st;
     HMG_CUDA_TRY(cudaStreamSynchronize(s));
     return HMG_OK;
 }

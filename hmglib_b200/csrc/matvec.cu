@@ -37,12 +37,13 @@ template <typename T>
 __global__ void k_fill_near(const int* blocks_r0, const int* blocks_c0, const int* blocks_m2,
                             const long long* near_off, const int* tfirst, const int* tlast,
                             const int* tile_r0, const int* tile_s, const int* tile_pstart,
-                            KernelSpec K, PointsView P, const double* bparam, T* out)
+                            KernelSpec K, PointsView P, const double* bparam, T* out, unsigned* top)
 {
     const int b = blockIdx.x;
     if (bparam) K.param = bparam[b];
     const int c0 = blocks_c0[b], m2 = blocks_m2[b];
     (void)blocks_r0;
+    unsigned largest = 0u;
     T* base = out + near_off[b];
     const int p0 = tile_pstart[tfirst[b]];
     for (int t = tfirst[b]; t <= tlast[b]; t++) {
@@ -50,9 +51,12 @@ __global__ void k_fill_near(const int* blocks_r0, const int* blocks_c0, const in
         T* dst = base + (size_t)(tile_pstart[t] - p0) * m2;
         for (int idx = threadIdx.x; idx < sp * m2; idx += blockDim.x) {
             int i = idx % sp, j = idx / sp;
-            dst[idx] = i < s ? (T)kernel_entry(K, P, tr + i, c0 + j) : (T)0;
+            const T v = i < s ? (T)kernel_entry(K, P, tr + i, c0 + j) : (T)0;
+            dst[idx] = v;
+            if constexpr (sizeof(T) == 4) largest = max(largest, magnitude(v));
         }
     }
+    if constexpr (sizeof(T) == 4) record_top(largest, top);
 }
 
 void free_near(hmg_matrix* h)
@@ -62,7 +66,6 @@ void free_near(hmg_matrix* h)
     dfree(h->near_off, h->stream);
     h->near_prec = -1;
     h->near_stored = 0;
-    h->stored_range = -1;
     h->desc_near_mode = -1;
     if (h->near_mode == HMG_NEAR_STORED) h->near_mode = HMG_NEAR_ONTHEFLY;
     free_tc(h);  // its BF16 near slices are copies of this storage
@@ -97,6 +100,7 @@ hmg_status fill_near(hmg_matrix* h, int precision)
     h->near_entries = entries;
     hmg_status st = dalloc(&h->near_off, (size_t)(nd > 0 ? nd : 1), s);
     if (st) return st;
+    HMG_CUDA_TRY(cudaMemsetAsync(h->stored_top, 0, sizeof(unsigned), s));
     if (nd > 0) {
         cudaError_t ce = cudaMalloc(&h->near_data, (size_t)tot * esz);
         if (ce != cudaSuccess) {
@@ -111,11 +115,11 @@ hmg_status fill_near(hmg_matrix* h, int precision)
         if (precision == HMG_PREC_FP64)
             k_fill_near<double><<<nd, 256, 0, s>>>(h->blk_r0, h->blk_c0, h->blk_m2, h->near_off,
                                                    h->blk_tfirst, h->blk_tlast, h->tile_r0, h->tile_s,
-                                                   h->tile_pstart, h->kspec, P, h->blk_param, (double*)h->near_data);
+                                                   h->tile_pstart, h->kspec, P, h->blk_param, (double*)h->near_data, nullptr);
         else
             k_fill_near<float><<<nd, 256, 0, s>>>(h->blk_r0, h->blk_c0, h->blk_m2, h->near_off,
                                                   h->blk_tfirst, h->blk_tlast, h->tile_r0, h->tile_s,
-                                                  h->tile_pstart, h->kspec, P, h->blk_param, (float*)h->near_data);
+                                                  h->tile_pstart, h->kspec, P, h->blk_param, (float*)h->near_data, h->stored_top);
         HMG_LAUNCH_CHECK();
     }
     HMG_CUDA_TRY(cudaStreamSynchronize(s));

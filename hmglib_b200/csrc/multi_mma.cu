@@ -131,8 +131,8 @@ template <int NT> struct FragB {
 // bits of an FP32 value), range[RANGE_T] whether an entry of t is too large.  The kernels
 // launched after them, which read these vectors, multiply with FP32 multiply-adds instead
 // (step_fma) where a vector lies outside.  No kernel reads what it records itself: its warps
-// would disagree.  The stored FP32 values are looked at once, at the first product
-// (ensure_stored_range).  Within the range, the sum of a pair, at most 512 products of a stored
+// would disagree.  The kernels that write the stored FP32 values record their largest
+// (stored_top: near field, U, V), and a load looks for them (scan_stored_top).  Within the range, the sum of a pair, at most 512 products of a stored
 // value below 2^40 and an entry of X or t below 2^78, is finite, and so is a sum over a block's
 // columns, whose entries of V are below 2^9; the parts lose what lies below 2^-133, at most
 // 2^-63 of a vector's and 2^-103 of the storage's largest value.
@@ -141,11 +141,13 @@ static constexpr unsigned STORED_LARGE = (127u + 40) << 23, STORED_SMALL = (127u
 static constexpr unsigned V_LARGE = (127u + 9) << 23;
 static constexpr int RANGE_T = 32;
 static_assert(MULTI_RANGE_WORDS == RANGE_T + 1, "the record's words");
-__device__ __forceinline__ bool too_large(float v) { return (__float_as_uint(v) & 0x7fffffffu) >= RANGE_LARGE; }
+__device__ __forceinline__ bool too_large(float v) { return magnitude(v) >= RANGE_LARGE; }
 // the same in every warp
-__device__ __forceinline__ bool out_of_range(const unsigned* range, int R)
+__device__ __forceinline__ bool out_of_range(const unsigned* range, int R, const unsigned* stored)
 {
     const int lane = threadIdx.x & 31;
+    const unsigned a = max(stored[0], stored[1]);
+    if (a >= STORED_LARGE || (a != 0u && a < STORED_SMALL) || stored[2] >= V_LARGE) return true;
     const unsigned top = lane < R ? range[lane] : 0u;
     return __any_sync(0xffffffffu, top >= RANGE_LARGE || (top != 0u && top < RANGE_SMALL));
 }
@@ -239,7 +241,7 @@ __global__ void k_gather_mma(const double* X, int ldx, int nrhs, const int* perm
         const int i = (int)(idx / R), j = (int)(idx - (long long)i * R);
         const float v = j < nrhs ? (float)X[perm2[i] + (size_t)j * ldx] : 0.0f;
         xm[idx] = v;
-        atomicMax(&top[j], __float_as_uint(v) & 0x7fffffffu);
+        atomicMax(&top[j], magnitude(v));
     }
     __syncthreads();
     // (read first: after a few CTAs hardly any has a larger one)
@@ -290,7 +292,7 @@ template <int NT> struct VtShape {
 template <int NT>
 __global__ void __launch_bounds__(VtShape<NT>::WARPS * 32, 1)
 k_vtx_mma(const VtTask* __restrict__ tasks, int nlarge, int nsmall, const float* __restrict__ xm,
-           float* __restrict__ tm, unsigned* range, int stored_ok)
+           float* __restrict__ tm, unsigned* range, const unsigned* stored)
 {
     typedef VtShape<NT> S;
     constexpr int R = S::R, NS = S::NS, WARPS = S::WARPS;
@@ -318,7 +320,7 @@ k_vtx_mma(const VtTask* __restrict__ tasks, int nlarge, int nsmall, const float*
         }
     };
     const int ntask = nlarge + nsmall;
-    const bool plain = !stored_ok || out_of_range(range, R);
+    const bool plain = out_of_range(range, R, stored);
     bool large = false;
 
     // producer: the lane's rows of the task (offsets from the block's V, which may pass 4 GiB,
@@ -645,7 +647,7 @@ template <int NT>
 __global__ void __launch_bounds__(TtShape<NT>::WARPS * 32, TtShape<NT>::CTAS)
 k_tile_mma(const PairDesc* __restrict__ desc, const int* tile_pair_start, const int* tile_r0, const int* tile_s,
             const int* perm1, const float* __restrict__ xm, const float* __restrict__ tm, const char* tbase, int nrhs,
-            double* Y, int ldy, int only_kind, const unsigned* range, int stored_ok)
+            double* Y, int ldy, int only_kind, const unsigned* range, const unsigned* stored)
 {
     typedef TtShape<NT> S;
     constexpr int R = S::R, NS = S::NS, SB = S::SB;
@@ -659,7 +661,7 @@ k_tile_mma(const PairDesc* __restrict__ desc, const int* tile_pair_start, const 
     char* ring = tt_smem + (size_t)warp * NS * S::STAGE;
     const uint32_t ring_s = static_cast<uint32_t>(__cvta_generic_to_shared(ring));
     const int pend = g < G ? tile_pair_start[t + 1] : 0;
-    const bool plain = !stored_ok || out_of_range(range, R) || range[RANGE_T] != 0u;
+    const bool plain = out_of_range(range, R, stored) || range[RANGE_T] != 0u;
 
     // producer: pair; within it the tier (0 FP32, 1 FP16, 2 FP8), the lane's next slice and
     // vector addresses, chunk columns left in the tier
@@ -873,83 +875,57 @@ k_tile_mma(const PairDesc* __restrict__ desc, const int* tile_pair_start, const 
 }
 
 // ---------------------------------------------------------------------------
-// the range of the stored FP32 values
+// the range of loaded FP32 values
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ unsigned largest(unsigned top, const uint4* p, long long n, int i0, int step)
+__device__ __forceinline__ unsigned largest16(const uint4* p, long long n, long long i, long long step)
 {
-    for (long long i = i0; i < n; i += step) {
+    unsigned top = 0u;
+    for (; i < n; i += step) {
         const uint4 v = ld_stream(p + i);
         top = max(max(top, v.x & 0x7fffffffu), max(v.y & 0x7fffffffu, max(v.z & 0x7fffffffu, v.w & 0x7fffffffu)));
     }
     return top;
 }
 
-__device__ __forceinline__ void record(unsigned top, unsigned* out)
+__global__ void k_near_top(const uint4* near, long long n16, unsigned* top)
 {
-    top = __reduce_max_sync(0xffffffffu, top);
-    if ((threadIdx.x & 31) == 0 && top > *static_cast<volatile unsigned*>(out)) atomicMax(out, top);
+    record_top(largest16(near, n16, blockIdx.x * (long long)blockDim.x + threadIdx.x, gridDim.x * (long long)blockDim.x), top);
 }
 
-// top[0]: the largest magnitude (bits) of the near field and of U, top[1]: of V
-__global__ void k_near_range(const uint4* near, long long n16, unsigned* top)
+// the FP32 terms of U and V, a CTA a block
+__global__ void k_far_top(int b0, const int* tfirst, const int* tlast, const int* tile_s, const int* tile_pstart,
+                          const int* blk_m2, const int* rank, const int* tier32, const int* tier16, int mixed,
+                          void* const* ptrU, void* const* ptrV, unsigned* top)
 {
-    record(largest(0u, near, n16, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x), top);
-}
-
-// (the FP32 terms; a warp a block)
-__global__ void k_far_range(int b0, int nb, const int* tfirst, const int* tlast, const int* tile_s, const int* tile_pstart,
-                            const int* blk_m2, const int* rank, const int* tier32, const int* tier16, int mixed,
-                            void* const* ptrU, void* const* ptrV, unsigned* top)
-{
-    const int lane = threadIdx.x & 31;
-    const int b = b0 + blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (b >= nb) return;
-    const int r = rank[b], r32 = mixed ? tier32[b] : r, r16 = mixed ? tier16[b] : 0;
+    const int b = b0 + blockIdx.x, r = rank[b], r32 = mixed ? tier32[b] : r, r16 = mixed ? tier16[b] : 0;
     if (r == 0) return;
     const long long bpr = 4ll * r32 + 2ll * r16 + (r - r32 - r16);
     unsigned u = 0u;
     for (int t = tfirst[b]; t <= tlast[b]; t++) {
         const char* slice = static_cast<const char*>(ptrU[b]) + (tile_pstart[t] - tile_pstart[tfirst[b]]) * bpr;
-        u = largest(u, reinterpret_cast<const uint4*>(slice), (long long)((tile_s[t] + 3) >> 2) * r32, lane, 32);
+        u = max(u, largest16(reinterpret_cast<const uint4*>(slice), (long long)((tile_s[t] + 3) >> 2) * r32, threadIdx.x, blockDim.x));
     }
-    record(u, top);
-    record(largest(0u, static_cast<const uint4*>(ptrV[b]), (long long)((blk_m2[b] + 3) >> 2) * r32, lane, 32), top + 1);
+    record_top(u, top + 1);
+    record_top(largest16(static_cast<const uint4*>(ptrV[b]), (long long)((blk_m2[b] + 3) >> 2) * r32, threadIdx.x, blockDim.x),
+               top + 2);
 }
 
-// Once per storage (8 GB: 1.4 ms, the time of one product): whether its FP32 values are in
-// the MMAs' range, an infinity or a NaN among them or none.
-static hmg_status ensure_stored_range(hmg_matrix* h)
+hmg_status scan_stored_top(hmg_matrix* h)
 {
-    if (h->stored_range >= 0) return HMG_OK;
     cudaStream_t s = h->stream;
-    hmg_status st;
-    unsigned* top = nullptr;
-    if ((st = dalloc(&top, 2, s))) return st;
-    unsigned found[2] = {0u, 0u};
-    const bool near = h->ndense > 0 && h->near_prec == HMG_PREC_FP32;
-    const bool mixed = h->far_prec == HMG_PREC_MIXED;
-    cudaError_t e = cudaMemsetAsync(top, 0, 2 * sizeof(unsigned), s);
-    if (e == cudaSuccess && near) {
-        const long long n16 = h->near_stored / 4;  // rows are padded to 16 bytes
-        k_near_range<<<(int)std::min<long long>(h->nsm * 8, ceil_div(n16, 256) + 1), 256, 0, s>>>(
-            static_cast<const uint4*>(h->near_data), n16, top);
-        e = cudaGetLastError();
+    HMG_CUDA_TRY(cudaMemsetAsync(h->stored_top, 0, 3 * sizeof(unsigned), s));
+    if (h->ndense > 0 && h->near_prec == HMG_PREC_FP32) {
+        const long long n16 = h->near_stored / 4;  // columns are padded to 16 bytes
+        k_near_top<<<(int)std::min<long long>(h->nsm * 8, (n16 + 255) / 256 + 1), 256, 0, s>>>(
+            static_cast<const uint4*>(h->near_data), n16, h->stored_top);
+        HMG_LAUNCH_CHECK();
     }
-    if (e == cudaSuccess && h->nblocks > h->ndense && h->far_prec >= 0) {
-        k_far_range<<<ceil_div(h->nblocks - h->ndense, 8), 256, 0, s>>>(
-            h->ndense, h->nblocks, h->blk_tfirst, h->blk_tlast, h->tile_s, h->tile_pstart, h->blk_m2, h->rank, h->tier32,
-            h->tier16, mixed ? 1 : 0, h->ptrU, h->ptrV, top);
-        e = cudaGetLastError();
+    if (h->nblocks > h->ndense && (h->far_prec == HMG_PREC_FP32 || h->far_prec == HMG_PREC_MIXED)) {
+        k_far_top<<<h->nblocks - h->ndense, 256, 0, s>>>(h->ndense, h->blk_tfirst, h->blk_tlast, h->tile_s, h->tile_pstart,
+                                                         h->blk_m2, h->rank, h->tier32, h->tier16,
+                                                         h->far_prec == HMG_PREC_MIXED ? 1 : 0, h->ptrU, h->ptrV, h->stored_top);
+        HMG_LAUNCH_CHECK();
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(found, top, sizeof(found), cudaMemcpyDeviceToHost, s);
-    dfree(top, s);
-    const cudaError_t done = cudaStreamSynchronize(s);
-    if (e == cudaSuccess) e = done;
-    if (e != cudaSuccess) {
-        set_error("hmg_matvec_multi: reading the range of the stored values failed: %s", cudaGetErrorString(e));
-        return HMG_ERR_CUDA;
-    }
-    h->stored_range = found[0] < STORED_LARGE && (found[0] == 0u || found[0] >= STORED_SMALL) && found[1] < V_LARGE;
     return HMG_OK;
 }
 
@@ -961,7 +937,7 @@ static hmg_status launch_tiles(hmg_matrix* h, const float* xm, const float* tm, 
     HMG_CUDA_TRY(cudaFuncSetAttribute(k_tile_mma<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, TtShape<NT>::SMEM));
     k_tile_mma<NT><<<h->ntiles, TtShape<NT>::WARPS * 32, TtShape<NT>::SMEM, h->stream>>>(
         static_cast<const PairDesc*>(h->tile_desc), h->tile_desc_start, h->tile_r0, h->tile_s, h->perm[0], xm, tm,
-        static_cast<const char*>(h->tbuf), nrhs, Y, ldy, only_kind, range, h->stored_range);
+        static_cast<const char*>(h->tbuf), nrhs, Y, ldy, only_kind, range, h->stored_top);
     HMG_LAUNCH_CHECK();
     return HMG_OK;
 }
@@ -974,7 +950,7 @@ static hmg_status launch_all(hmg_matrix* h, const float* xm, float* tm, int nrhs
         HMG_CUDA_TRY(cudaFuncSetAttribute(k_vtx_mma<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, VtShape<NT>::SMEM));
         const int grid = std::min(h->nsm, nl + ceil_div(ns, VtShape<NT>::WARPS));
         k_vtx_mma<NT><<<grid, VtShape<NT>::WARPS * 32, VtShape<NT>::SMEM, h->stream>>>(static_cast<const VtTask*>(h->vt_tasks), nl,
-                                                                              ns, xm, tm, range, h->stored_range);
+                                                                              ns, xm, tm, range, h->stored_top);
         HMG_LAUNCH_CHECK();
     }
     return launch_tiles<NT>(h, xm, tm, nrhs, Y, ldy, -1, range);
@@ -985,7 +961,7 @@ hmg_status matvec_multi_mma(hmg_matrix* h, int nrhs, const double* X, int ldx, d
     cudaStream_t s = h->stream;
     hmg_status st;
     const int nt = (nrhs + 7) / 8, R = 8 * nt;
-    if ((st = ensure_desc(h, 4)) || (st = ensure_vt(h)) || (st = ensure_stored_range(h))) return st;
+    if ((st = ensure_desc(h, 4)) || (st = ensure_vt(h))) return st;
     float* xm = nullptr;
     float* tm = nullptr;
     // the range record sits behind xm
@@ -1021,8 +997,8 @@ hmg_status near_multi32(hmg_matrix* h, const double* X, int ldx, int nrhs, float
 {
     // a product in another near-field mode or arithmetic may have left other descriptors, and
     // one that ran out of memory none
-    hmg_status st;
-    if ((st = ensure_desc(h, 4)) || (st = ensure_stored_range(h))) return st;
+    hmg_status st = ensure_desc(h, 4);
+    if (st) return st;
     unsigned* range = reinterpret_cast<unsigned*>(xm + (size_t)h->n[1] * 32);
     HMG_CUDA_TRY(cudaMemsetAsync(range, 0, MULTI_RANGE_WORDS * sizeof(unsigned), h->stream));
     k_gather_mma<<<ceil_div((long long)h->n[1] * 32, 256), 256, 0, h->stream>>>(X, ldx, nrhs, h->perm[1], h->n[1], 32,

@@ -48,6 +48,15 @@ __device__ __forceinline__ uint4 ld_stream(const void* p)
         : "l"(p));
     return v;
 }
+// the magnitude of an FP32 value as bits that compare like it (infinities and NaN on top)
+__device__ __forceinline__ unsigned magnitude(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+// *out = max(*out, the warp's tops), by all its lanes
+__device__ __forceinline__ void record_top(unsigned top, unsigned* out)
+{
+    top = __reduce_max_sync(0xffffffffu, top);
+    // (read first: after a few warps hardly any has a larger one)
+    if ((threadIdx.x & 31) == 0 && top > *static_cast<volatile unsigned*>(out)) atomicMax(out, top);
+}
 // longest pair a tile kernel's warp takes whole (why: k_count_chunks in matvec.cu)
 static constexpr int TILE_CHUNK = 256;
 // largest rank the streaming V^T x kernel accepts

@@ -91,7 +91,7 @@ def test_both_ends_of_the_range(hmg, cuda, storage, log2):
 
 @pytest.mark.parametrize("reg", [3.39e38, 1e39, -1e39, 1e13])
 @pytest.mark.parametrize("storage", ["fp32", "mixed"])
-def test_stored_values_that_do_not_split(hmg, cuda, storage, reg):
+def test_stored_values_that_do_not_split(hmg, cuda, tmp_path, storage, reg):
     """A regularization near, beyond and far below the FP32 limit: the stored diagonal is huge or
     infinite, and the multi-vector products have the single-vector product's finite, infinite
     and undefined entries (one vector is zero at some points) and its values to 1e-6."""
@@ -116,6 +116,14 @@ def test_stored_values_that_do_not_split(hmg, cuda, storage, reg):
         fin = np.isfinite(one)
         if fin.any():
             assert rel_err(a[fin], one[fin]) < 1e-6
+    # the same through a file
+    H.save(str(tmp_path / "h"))
+    L = hmg.load(str(tmp_path / "h"))
+    Z = torch.empty_like(Y)
+    L.matvec_multi(X, Z)
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(Z.cpu().numpy(), Y.cpu().numpy())
+    L.close()
     # another regularization, the same handle: back to finite products
     H.set_kernel(GAUSS, 0.05, 0.5)
     H.precompute_aca(64, 1e-8, hmg.PREC_MIXED if storage == "mixed" else hmg.PREC_FP32)
