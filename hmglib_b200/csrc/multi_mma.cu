@@ -30,8 +30,8 @@
 // Measured at N = 2^17 (uniform 3D, Matern, mixed storage, 8.0 GB: 1.23 ms at the copy
 // peak) against the CUDA-core kernels (packed FP32 multiply-adds) this replaces: 8
 // vectors 3.42 ms (7.18), 16 5.10 (9.45), 24 6.34 (14.1), 32 8.41 (14.1); with the two TF32
-// parts 2.77, 3.95, 5.16 and 6.94.  Bound by instruction issue and the latency of the MMA
-// chains, not by memory.
+// parts 2.77, 3.95, 5.16 and 6.94.  Bound by instruction issue (8 vectors: 52-61 % active) and
+// the latency of the MMA chains (32: tensor pipe 40-53 % busy), not by memory.
 #include <cuda_fp16.h>
 #include <cuda_fp8.h>
 
