@@ -229,9 +229,10 @@ hmg_status hmg_group_offsets(hmg_matrix* h, int set, int64_t* offsets);
 
 /* Y = H X for 1 <= nrhs <= 64 vectors: X (n2 x nrhs) and Y (n1 x nrhs) are device
  * FP64 column-major with leading dimensions ldx >= n2, ldy >= n1, caller order.  The
- * stored H-matrix is read once per 32 vectors (FP32 / FP64 storage with a stored near
- * field; otherwise one product per vector), once for all 64 with tensor-core operands
- * (hmg_build_tensor_core_operands).  Same arithmetic as hmg_matvec;
+ * stored H-matrix is read once per 32 vectors (FP32, mixed or FP64 storage with a stored
+ * near field; otherwise, and in FP64 arithmetic over FP32 or mixed storage, one product per
+ * vector), once for all 64 with tensor-core operands (hmg_build_tensor_core_operands).
+ * Without those the precision is that of hmg_matvec, the order of the sums is not;
  * asynchronous on the handle's stream.  No reference counterpart (the reference
  * multiplies one vector per apply_h_matrix_mvp call, hmglib.cu:271-286). */
 hmg_status hmg_matvec_multi(hmg_matrix* h, int nrhs, const double* X, int ldx, double* Y, int ldy);
